@@ -51,12 +51,26 @@ __device__ __forceinline__ void load8f(const float* p, float (&f)[8]) {
   f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
+// Norm scale as the caller holds it: an fp32 parameter, or the bf16 compute copy that the parameter store keeps of
+// every parameter.
+struct NormScale {
+  const void* p;
+  int bf16;
+  __device__ __forceinline__ explicit operator bool() const { return p != nullptr; }
+};
+__device__ __forceinline__ void load8w(const NormScale& w, int col, float (&f)[8]) {
+  if (w.bf16)
+    unpack8(*reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(w.p) + col), f);
+  else
+    load8f(reinterpret_cast<const float*>(w.p) + col, f);
+}
+
 // ------------------------------------------------------------------------------------------------
 // RMSNorm forward: optionally res_out = x + delta first.  One warp per row, H % 8 == 0.
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                   const float* __restrict__ w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
+                   NormScale w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
                    float* __restrict__ rstd_out, int rows, int H, float eps) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -90,7 +104,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     for (int v = lane; v < nvec; v += 32) {
       float f[8], wv[8];
       unpack8(src[v], f);
-      load8f(w + v * 8, wv);
+      load8w(w, v * 8, wv);
 #pragma unroll
       for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * wv[i];
       yr[v] = pack8(f);
@@ -103,7 +117,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 template <int NV>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                       const float* __restrict__ w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
+                       NormScale w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
                        float* __restrict__ rstd_out, int rows, float eps) {
   constexpr int H = NV * 256;
   const int lane = threadIdx.x & 31;
@@ -144,7 +158,7 @@ rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
     for (int j = 0; j < NV; ++j) {
       float f[8], wv[8];
       unpack8(raw[j], f);
-      load8f(w + (lane + 32 * j) * 8, wv);
+      load8w(w, (lane + 32 * j) * 8, wv);
 #pragma unroll
       for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * wv[i];
       yr[lane + 32 * j] = pack8(f);
@@ -156,7 +170,7 @@ rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
 // once instead of one warp walking it.
 __global__ void __launch_bounds__(256)
 rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                       const float* __restrict__ w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
+                       NormScale w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
                        float* __restrict__ rstd_out, int H, float eps) {
   __shared__ float part[8];
   b200::pdl_launch_dependents();   // no-ops unless launched as a dependent (decode steps)
@@ -195,7 +209,7 @@ rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
   for (int v = threadIdx.x; v < nvec; v += 256) {  // a thread re-reads only what it wrote itself
     float f[8], wv[8];
     unpack8(src[v], f);
-    load8f(w + v * 8, wv);
+    load8w(w, v * 8, wv);
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * wv[i];
     yr[v] = pack8(f);
@@ -226,7 +240,7 @@ splitk_finish_kernel(float* __restrict__ ws, __nv_bfloat16* __restrict__ out, lo
 // partials in shared memory and issues one fp32 atomicAdd per column.
 template <int NV>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, (NV == 8 ? 2 : 1))
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
+rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, NormScale w,
                    const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dy,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
                    int rows, int H) {
@@ -265,7 +279,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
         float f[8], g[8], wv[8];
         unpack8(xraw[j], f);
         unpack8(graw[j], g);
-        load8f(w + (lane + 32 * j) * 8, wv);
+        load8w(w, (lane + 32 * j) * 8, wv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) dot += g[i] * wv[i] * f[i] * rstd;
       }
@@ -276,7 +290,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
         float f[8], g[8], wv[8];
         unpack8(xr[v], f);
         unpack8(gr[v], g);
-        load8f(w + v * 8, wv);
+        load8w(w, v * 8, wv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) dot += g[i] * wv[i] * f[i] * rstd;
       }
@@ -285,7 +299,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
         float f[8], g[8], wv[8];
         unpack8(xr[v], f);
         unpack8(gr[v], g);
-        load8f(w + v * 8, wv);
+        load8w(w, v * 8, wv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) dot += g[i] * wv[i] * f[i] * rstd;
       }
@@ -300,7 +314,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
         float f[8], g[8], wv[8], o[8];
         unpack8(kInRegs ? xraw[j < NRAW ? j : 0] : xr[v], f);
         unpack8(kInRegs ? graw[j < NRAW ? j : 0] : gr[v], g);
-        load8f(w + v * 8, wv);
+        load8w(w, v * 8, wv);
         float r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         if (rr) unpack8(rr[v], r);
 #pragma unroll
@@ -316,7 +330,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
         float f[8], g[8], wv[8], o[8];
         unpack8(xr[v], f);
         unpack8(gr[v], g);
-        load8f(w + v * 8, wv);
+        load8w(w, v * 8, wv);
         float r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         if (rr) unpack8(rr[v], r);
 #pragma unroll
@@ -348,7 +362,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
 // through shared memory per row, double buffered by parity), which keeps loads in flight all the time.
 template <int VEC, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
-rmsnorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
+rmsnorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ x, NormScale w,
                         const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dy,
                         const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw, int rows, int H) {
@@ -360,7 +374,7 @@ rmsnorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ x, const float* __rest
   float wv[VEC][8], acc[VEC][8];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
-    load8f(w + (t + v * THREADS) * 8, wv[v]);
+    load8w(w, (t + v * THREADS) * 8, wv[v]);
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
   }
@@ -460,9 +474,9 @@ __device__ __forceinline__ float group_sum(float v, int lph) {
 
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride, __nv_bfloat16* __restrict__ out,
-                       long long out_stride, const float* __restrict__ w, const int* __restrict__ positions,
+                       long long out_stride, NormScale w, const int* __restrict__ positions,
                        float* __restrict__ rstd_out, long long tokens, int heads, int D, float eps, float log2_theta,
-                       int rope, int lph, const float* __restrict__ w2, int heads_first) {
+                       int rope, int lph, NormScale w2, int heads_first) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int hpw = 32 / lph;
@@ -474,8 +488,8 @@ qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride
 #pragma unroll
   for (int i = 0; i < 4; ++i) inv_freq[i] = exp2f(-log2_theta * (2.f * (float)(l * 4 + i)) / (float)D);
   // the norm scales are weights (no predecessor writes them): they are read before the wait for the predecessor
-  if (w && has_cols) load8f(w + l * 8, wv);
-  if (w2 && has_cols) load8f(w2 + l * 8, wv2);
+  if (w && has_cols) load8w(w, l * 8, wv);
+  if (w2 && has_cols) load8w(w2, l * 8, wv2);
   b200::pdl_launch_dependents();   // no-ops unless launched as a dependent (decode steps)
   b200::pdl_wait();
   const long long groups = (total + hpw - 1) / hpw;
@@ -517,10 +531,10 @@ qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride,
                        const __nv_bfloat16* __restrict__ dout, long long dout_stride,
-                       __nv_bfloat16* __restrict__ din, long long din_stride, const float* __restrict__ w,
+                       __nv_bfloat16* __restrict__ din, long long din_stride, NormScale w,
                        const int* __restrict__ positions, const float* __restrict__ rstd_in,
                        float* __restrict__ dw, long long tokens, int heads, int D, float log2_theta, int rope,
-                       int lph, const float* __restrict__ w2, float* __restrict__ dw2, int heads_first) {
+                       int lph, NormScale w2, float* __restrict__ dw2, int heads_first) {
   __shared__ float dw_smem[512];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -533,8 +547,8 @@ qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride
   float inv_freq[4], wv[8] = {0, 0, 0, 0, 0, 0, 0, 0}, wv2[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
   for (int i = 0; i < 4; ++i) inv_freq[i] = exp2f(-log2_theta * (2.f * (float)(l * 4 + i)) / (float)D);
-  if (w && has_cols) load8f(w + l * 8, wv);
-  if (w2 && has_cols) load8f(w2 + l * 8, wv2);
+  if (w && has_cols) load8w(w, l * 8, wv);
+  if (w2 && has_cols) load8w(w2, l * 8, wv2);
   float dw_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, dw_acc2[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   const long long groups = (total + hpw - 1) / hpw;
   for (long long gidx = (long long)blockIdx.x * kWarpsPerBlock + warp; gidx < groups;
@@ -1048,20 +1062,20 @@ inline int grid_for(long long work_items, int block, int per_sm = 8) {
 #define STREAM(s) reinterpret_cast<cudaStream_t>(s)
 #define LAST_ERR() static_cast<int>(cudaGetLastError())
 
-extern "C" int b200_rmsnorm_fwd(const void* x, const void* delta, const void* w, void* res_out, void* y, void* rstd,
+extern "C" int b200_rmsnorm_fwd(const void* x, const void* delta, const void* w, int w_bf16, void* res_out, void* y, void* rstd,
                                 int rows, int H, float eps, void* stream) {
   if (H % 8) return -2;
   if (rows > 0 && rows <= 512) {
     // few rows = a decode step: launched as a dependent so that it is resident when its predecessor ends
     return static_cast<int>(b200host::launch_kernel(
         rmsnorm_fwd_row_kernel, dim3(rows), dim3(256), 0, STREAM(stream), b200host::pdl_enabled() != 0,
-        (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, (const float*)w, (__nv_bfloat16*)res_out,
+        (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, NormScale{w, w_bf16}, (__nv_bfloat16*)res_out,
         (__nv_bfloat16*)y, (float*)rstd, H, eps));
   }
   const int grid = grid_for((long long)rows, kWarpsPerBlock, 8);
 #define RMS_FWD(NV)                                                                                         \
   rmsnorm_fwd_reg_kernel<NV><<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(                             \
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, (const float*)w, (__nv_bfloat16*)res_out,       \
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, NormScale{w, w_bf16}, (__nv_bfloat16*)res_out,       \
       (__nv_bfloat16*)y, (float*)rstd, rows, eps);                                                         \
   return LAST_ERR()
   switch (H) {
@@ -1072,17 +1086,17 @@ extern "C" int b200_rmsnorm_fwd(const void* x, const void* delta, const void* w,
   }
 #undef RMS_FWD
   rmsnorm_fwd_kernel<<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, (const float*)w, (__nv_bfloat16*)res_out,
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, NormScale{w, w_bf16}, (__nv_bfloat16*)res_out,
       (__nv_bfloat16*)y, (float*)rstd, rows, H, eps);
   return LAST_ERR();
 }
-extern "C" int b200_rmsnorm_bwd(const void* x, const void* w, const void* rstd, const void* dy, const void* dres,
+extern "C" int b200_rmsnorm_bwd(const void* x, const void* w, int w_bf16, const void* rstd, const void* dy, const void* dres,
                                 void* dx, void* dw, int rows, int H, void* stream) {
   if (H % 8 || H * 4 > 48 * 1024) return -2;
   if (H == 4096 || H == 8192) {   // narrower rows: the warp-per-row kernel below measured faster
 #define RMS_BWD_COLS(VEC, THREADS, MINB)                                                                        \
   rmsnorm_bwd_cols_kernel<VEC, THREADS, MINB><<<grid_for((long long)rows, 1, MINB), THREADS, 0, STREAM(stream)>>>( \
-      (const __nv_bfloat16*)x, (const float*)w, (const float*)rstd, (const __nv_bfloat16*)dy,                   \
+      (const __nv_bfloat16*)x, NormScale{w, w_bf16}, (const float*)rstd, (const __nv_bfloat16*)dy,                   \
       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (float*)dw, rows, H)
     if (H == 4096) RMS_BWD_COLS(2, 256, 2);
     else RMS_BWD_COLS(2, 512, 1);
@@ -1092,7 +1106,7 @@ extern "C" int b200_rmsnorm_bwd(const void* x, const void* w, const void* rstd, 
   const int grid = grid_for((long long)rows, kWarpsPerBlock, 2);
 #define RMS_BWD(NV)                                                                                     \
   rmsnorm_bwd_kernel<NV><<<grid, kWarpsPerBlock * 32, H * sizeof(float), STREAM(stream)>>>(              \
-      (const __nv_bfloat16*)x, (const float*)w, (const float*)rstd, (const __nv_bfloat16*)dy,            \
+      (const __nv_bfloat16*)x, NormScale{w, w_bf16}, (const float*)rstd, (const __nv_bfloat16*)dy,            \
       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (float*)dw, rows, H)
   switch (H) {
     case 256: RMS_BWD(1); break;
@@ -1111,20 +1125,20 @@ static int lanes_per_head(int D) {
   return lph;
 }
 extern "C" int b200_qknorm_rope_fwd(const void* in, long long in_stride, void* out, long long out_stride,
-                                    const void* w, const void* positions, void* rstd, long long tokens, int heads,
+                                    const void* w, int w_bf16, const void* positions, void* rstd, long long tokens, int heads,
                                     int D, float eps, float theta, int rope, void* stream) {
   if (D % 8 || D > 256) return -2;
   const int lph = lanes_per_head(D);
   const int grid = grid_for((tokens * heads + 32 / lph - 1) / (32 / lph), kWarpsPerBlock, 8);
   return static_cast<int>(b200host::launch_kernel(qknorm_rope_fwd_kernel, dim3(grid), dim3(kWarpsPerBlock * 32), 0,
                                                   STREAM(stream), tokens <= 512 && b200host::pdl_enabled() != 0,
-      (const __nv_bfloat16*)in, in_stride, (__nv_bfloat16*)out, out_stride, (const float*)w, (const int*)positions,
-      (float*)rstd, tokens, heads, D, eps, log2f(theta), rope, lph, nullptr, heads));
+      (const __nv_bfloat16*)in, in_stride, (__nv_bfloat16*)out, out_stride, NormScale{w, w_bf16}, (const int*)positions,
+      (float*)rstd, tokens, heads, D, eps, log2f(theta), rope, lph, NormScale{nullptr, 0}, heads));
 }
 // Query and key heads of a packed projection in one launch: the first heads_q heads use wq, the next heads_k use wk
 // (both or neither given); rstd is [tokens, heads_q + heads_k].
 extern "C" int b200_qknorm_rope_fwd_qk(const void* in, long long in_stride, void* out, long long out_stride,
-                                       const void* wq, const void* wk, const void* positions, void* rstd,
+                                       const void* wq, const void* wk, int w_bf16, const void* positions, void* rstd,
                                        long long tokens, int heads_q, int heads_k, int D, float eps, float theta,
                                        int rope, void* stream) {
   if (D % 8 || D > 256 || (wq == nullptr) != (wk == nullptr)) return -2;
@@ -1133,11 +1147,11 @@ extern "C" int b200_qknorm_rope_fwd_qk(const void* in, long long in_stride, void
   const int grid = grid_for((tokens * heads + 32 / lph - 1) / (32 / lph), kWarpsPerBlock, 8);
   return static_cast<int>(b200host::launch_kernel(qknorm_rope_fwd_kernel, dim3(grid), dim3(kWarpsPerBlock * 32), 0,
                                                   STREAM(stream), tokens <= 512 && b200host::pdl_enabled() != 0,
-      (const __nv_bfloat16*)in, in_stride, (__nv_bfloat16*)out, out_stride, (const float*)wq, (const int*)positions,
-      (float*)rstd, tokens, heads, D, eps, log2f(theta), rope, lph, (const float*)wk, heads_q));
+      (const __nv_bfloat16*)in, in_stride, (__nv_bfloat16*)out, out_stride, NormScale{wq, w_bf16}, (const int*)positions,
+      (float*)rstd, tokens, heads, D, eps, log2f(theta), rope, lph, NormScale{wk, w_bf16}, heads_q));
 }
 extern "C" int b200_qknorm_rope_bwd(const void* in, long long in_stride, const void* dout, long long dout_stride,
-                                    void* din, long long din_stride, const void* w, const void* positions,
+                                    void* din, long long din_stride, const void* w, int w_bf16, const void* positions,
                                     const void* rstd, void* dw, long long tokens, int heads, int D, float theta,
                                     int rope, void* stream) {
   if (D % 8 || D > 256) return -2;
@@ -1145,13 +1159,13 @@ extern "C" int b200_qknorm_rope_bwd(const void* in, long long in_stride, const v
   const int grid = grid_for((tokens * heads + 32 / lph - 1) / (32 / lph), kWarpsPerBlock, 4);
   qknorm_rope_bwd_kernel<<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(
       (const __nv_bfloat16*)in, in_stride, (const __nv_bfloat16*)dout, dout_stride, (__nv_bfloat16*)din, din_stride,
-      (const float*)w, (const int*)positions, (const float*)rstd, (float*)dw, tokens, heads, D, log2f(theta), rope,
-      lph, nullptr, nullptr, heads);
+      NormScale{w, w_bf16}, (const int*)positions, (const float*)rstd, (float*)dw, tokens, heads, D, log2f(theta), rope,
+      lph, NormScale{nullptr, 0}, nullptr, heads);
   return LAST_ERR();
 }
 extern "C" int b200_qknorm_rope_bwd_qk(const void* in, long long in_stride, const void* dout, long long dout_stride,
                                        void* din, long long din_stride, const void* wq, const void* wk,
-                                       const void* positions, const void* rstd, void* dwq, void* dwk, long long tokens,
+                                       int w_bf16, const void* positions, const void* rstd, void* dwq, void* dwk, long long tokens,
                                        int heads_q, int heads_k, int D, float theta, int rope, void* stream) {
   if (D % 8 || D > 256 || (wq == nullptr) != (wk == nullptr)) return -2;
   const int heads = heads_q + heads_k;
@@ -1159,8 +1173,8 @@ extern "C" int b200_qknorm_rope_bwd_qk(const void* in, long long in_stride, cons
   const int grid = grid_for((tokens * heads + 32 / lph - 1) / (32 / lph), kWarpsPerBlock, 4);
   qknorm_rope_bwd_kernel<<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(
       (const __nv_bfloat16*)in, in_stride, (const __nv_bfloat16*)dout, dout_stride, (__nv_bfloat16*)din, din_stride,
-      (const float*)wq, (const int*)positions, (const float*)rstd, (float*)dwq, tokens, heads, D, log2f(theta), rope,
-      lph, (const float*)wk, (float*)dwk, heads_q);
+      NormScale{wq, w_bf16}, (const int*)positions, (const float*)rstd, (float*)dwq, tokens, heads, D, log2f(theta), rope,
+      lph, NormScale{wk, w_bf16}, (float*)dwk, heads_q);
   return LAST_ERR();
 }
 extern "C" int b200_swiglu_fwd(const void* gu, void* h, long long rows, int I, void* stream) {

@@ -80,16 +80,16 @@ def _declare(lib: ctypes.CDLL) -> None:
 
     sig("b200_gemm_bf16", c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_ll, c_ll, c_ll,
         c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p)
-    sig("b200_rmsnorm_fwd", c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p)
-    sig("b200_rmsnorm_bwd", c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p)
-    sig("b200_qknorm_rope_fwd", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int,
+    sig("b200_rmsnorm_fwd", c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p)
+    sig("b200_rmsnorm_bwd", c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p)
+    sig("b200_qknorm_rope_fwd", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_int, c_void_p, c_void_p, c_ll, c_int, c_int,
         c_float, c_float, c_int, c_void_p)
-    sig("b200_qknorm_rope_bwd", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p,
-        c_ll, c_int, c_int, c_float, c_int, c_void_p)
-    sig("b200_qknorm_rope_fwd_qk", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_ll, c_int,
-        c_int, c_int, c_float, c_float, c_int, c_void_p)
-    sig("b200_qknorm_rope_bwd_qk", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p,
-        c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_float, c_int, c_void_p)
+    sig("b200_qknorm_rope_bwd", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_int, c_void_p, c_void_p,
+        c_void_p, c_ll, c_int, c_int, c_float, c_int, c_void_p)
+    sig("b200_qknorm_rope_fwd_qk", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_ll,
+        c_int, c_int, c_int, c_float, c_float, c_int, c_void_p)
+    sig("b200_qknorm_rope_bwd_qk", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_void_p,
+        c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_float, c_int, c_void_p)
     sig("b200_swiglu_fwd", c_void_p, c_void_p, c_ll, c_int, c_void_p)
     sig("b200_swiglu_bwd", c_void_p, c_void_p, c_void_p, c_ll, c_int, c_void_p)
     sig("b200_sigmoid_gate_fwd", c_void_p, c_void_p, c_void_p, c_ll, c_void_p)
@@ -393,6 +393,15 @@ def _splitk_workspace(numel: int, device: torch.device) -> torch.Tensor:
     return ws
 
 
+def _scale_is_bf16(*scales: torch.Tensor | None) -> int:
+    """Norm scales are fp32 parameters or the bf16 compute copies of a parameter store; the kernels read either."""
+
+    kinds = {w.dtype for w in scales if w is not None}
+    if len(kinds) > 1 or not kinds <= {torch.float32, torch.bfloat16}:
+        raise KernelError(f"norm scales must share one of fp32 and bf16, got {sorted(map(str, kinds))}")
+    return int(torch.bfloat16 in kinds)
+
+
 def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float, delta: torch.Tensor | None = None):
     """Returns ``(y, rstd, residual)``; ``residual = x + delta`` when ``delta`` is given, else ``x``."""
 
@@ -402,7 +411,7 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float, delta: torch.Tenso
     y = torch.empty_like(x)
     rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
     res = torch.empty_like(x) if delta is not None else None
-    rc = lib.b200_rmsnorm_fwd(x.data_ptr(), _ptr(delta), w.data_ptr(), _ptr(res), y.data_ptr(), rstd.data_ptr(), rows, H,
+    rc = lib.b200_rmsnorm_fwd(x.data_ptr(), _ptr(delta), w.data_ptr(), _scale_is_bf16(w), _ptr(res), y.data_ptr(), rstd.data_ptr(), rows, H,
                               eps, _stream())
     _check(rc, "b200_rmsnorm_fwd")
     return y, rstd, (res if res is not None else x)
@@ -416,7 +425,7 @@ def rmsnorm_bwd(x: torch.Tensor, w: torch.Tensor, rstd: torch.Tensor, dy: torch.
     H = x.shape[-1]
     rows = x.numel() // H
     dx = torch.empty_like(x)
-    rc = lib.b200_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dy.data_ptr(), _ptr(dres), dx.data_ptr(),
+    rc = lib.b200_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), _scale_is_bf16(w), rstd.data_ptr(), dy.data_ptr(), _ptr(dres), dx.data_ptr(),
                               dw.data_ptr(), rows, H, _stream())
     _check(rc, "b200_rmsnorm_bwd")
     return dx
@@ -430,7 +439,7 @@ def qknorm_rope_fwd(inp: torch.Tensor, out: torch.Tensor, w: torch.Tensor | None
     tokens = inp.shape[0]
     rstd = torch.empty(tokens * heads, dtype=torch.float32, device=inp.device) if w is not None else None
     rc = lib.b200_qknorm_rope_fwd(inp.data_ptr(), inp.stride(0), out.data_ptr(), out.stride(0), _ptr(w),
-                                  positions.data_ptr(), _ptr(rstd), tokens, heads, head_dim, eps, theta, int(rope),
+                                  _scale_is_bf16(w), positions.data_ptr(), _ptr(rstd), tokens, heads, head_dim, eps, theta, int(rope),
                                   _stream())
     _check(rc, "b200_qknorm_rope_fwd")
     return rstd
@@ -441,7 +450,7 @@ def qknorm_rope_bwd(inp: torch.Tensor, dout: torch.Tensor, din: torch.Tensor, w:
                     head_dim: int, theta: float, rope: bool) -> None:
     lib = load()
     rc = lib.b200_qknorm_rope_bwd(inp.data_ptr(), inp.stride(0), dout.data_ptr(), dout.stride(0), din.data_ptr(),
-                                  din.stride(0), _ptr(w), positions.data_ptr(), _ptr(rstd), _ptr(dw), inp.shape[0],
+                                  din.stride(0), _ptr(w), _scale_is_bf16(w), positions.data_ptr(), _ptr(rstd), _ptr(dw), inp.shape[0],
                                   heads, head_dim, theta, int(rope), _stream())
     _check(rc, "b200_qknorm_rope_bwd")
 
@@ -457,7 +466,7 @@ def qknorm_rope_fwd_qk(inp: torch.Tensor, out: torch.Tensor, wq, wk, positions: 
     if wq is not None:
         rstd = torch.empty(tokens * (heads_q + heads_k), dtype=torch.float32, device=inp.device)
     rc = lib.b200_qknorm_rope_fwd_qk(inp.data_ptr(), inp.stride(0), out.data_ptr(), out.stride(0), _ptr(wq), _ptr(wk),
-                                     positions.data_ptr(), _ptr(rstd), tokens, heads_q, heads_k, head_dim, eps, theta,
+                                     _scale_is_bf16(wq, wk), positions.data_ptr(), _ptr(rstd), tokens, heads_q, heads_k, head_dim, eps, theta,
                                      int(rope), _stream())
     _check(rc, "b200_qknorm_rope_fwd_qk")
     return rstd
@@ -467,7 +476,7 @@ def qknorm_rope_bwd_qk(inp: torch.Tensor, dout: torch.Tensor, din: torch.Tensor,
                        rstd, dwq, dwk, heads_q: int, heads_k: int, head_dim: int, theta: float, rope: bool) -> None:
     lib = load()
     rc = lib.b200_qknorm_rope_bwd_qk(inp.data_ptr(), inp.stride(0), dout.data_ptr(), dout.stride(0), din.data_ptr(),
-                                     din.stride(0), _ptr(wq), _ptr(wk), positions.data_ptr(), _ptr(rstd), _ptr(dwq),
+                                     din.stride(0), _ptr(wq), _ptr(wk), _scale_is_bf16(wq, wk), positions.data_ptr(), _ptr(rstd), _ptr(dwq),
                                      _ptr(dwk), inp.shape[0], heads_q, heads_k, head_dim, theta, int(rope), _stream())
     _check(rc, "b200_qknorm_rope_bwd_qk")
 

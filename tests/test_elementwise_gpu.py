@@ -36,6 +36,33 @@ def test_rmsnorm_fwd_bwd(H, rows):
     assert torch.allclose(dw, wr.grad, atol=5e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("H", [128, 768, 2048, 4096])
+@pytest.mark.parametrize("rows", [3, 600])
+def test_norm_scales_are_read_in_the_precision_they_are_held_in(H, rows):
+    """The parameter store holds norm scales as bf16 compute copies: the kernels give bit for bit what they give for
+    the same values in fp32, for RMSNorm and for the QK-norm, forward and backward."""
+
+    from research_b200.ops import native
+
+    x, dy = _bf((rows, H), 21), _bf((rows, H), 22)
+    wb = (torch.rand(H, device="cuda") + 0.5).to(torch.bfloat16)
+    got = []
+    for w in (wb, wb.float()):
+        y, rstd, _ = native.rmsnorm_fwd(x, w, 1e-6)
+        out = torch.empty_like(x)
+        r = native.qknorm_rope_fwd_qk(x, out, w[:64], w[64:128], torch.arange(rows, device="cuda", dtype=torch.int32), 1,
+                                      1, 64, 1e-6, 10000.0, True)
+        din, dq, dk = torch.zeros_like(x), torch.zeros(64, device="cuda"), torch.zeros(64, device="cuda")
+        native.qknorm_rope_bwd_qk(x, dy, din, w[:64], w[64:128], torch.arange(rows, device="cuda", dtype=torch.int32),
+                                  r, dq, dk, 1, 1, 64, 10000.0, True)
+        dx = native.rmsnorm_bwd(x, w, rstd, dy, torch.zeros(H, device="cuda"))
+        got.append((y, out[:, :128], din[:, :128], dx))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    with pytest.raises(native.KernelError):
+        native.rmsnorm_fwd(x, wb.half(), 1e-6)
+
+
 def _rope_ref(x, pos, theta):
     D = x.shape[-1]
     inv = theta ** (-torch.arange(0, D, 2, device=x.device, dtype=torch.float32) / D)
