@@ -51,26 +51,26 @@ __device__ __forceinline__ void load8f(const float* p, float (&f)[8]) {
   f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
-// Norm scale as the caller holds it: an fp32 parameter, or the bf16 compute copy that the parameter store keeps of
-// every parameter.
-struct NormScale {
-  const void* p;
-  int bf16;
-  __device__ __forceinline__ explicit operator bool() const { return p != nullptr; }
-};
-__device__ __forceinline__ void load8w(const NormScale& w, int col, float (&f)[8]) {
-  if (w.bf16)
-    unpack8(*reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(w.p) + col), f);
-  else
-    load8f(reinterpret_cast<const float*>(w.p) + col, f);
+// Norm scales come as the caller holds them: an fp32 parameter, or the bf16 compute copy that the parameter store keeps
+// of every parameter.  The kernels are templates on that type (a test at each load cost the forward kernel a fifth of
+// its rate at 2999 rows of 4096).
+__device__ __forceinline__ void load8w(const float* w, float (&f)[8]) { load8f(w, f); }
+__device__ __forceinline__ void load8w(const __nv_bfloat16* w, float (&f)[8]) {
+  unpack8(*reinterpret_cast<const uint4*>(w), f);
+}
+// four consecutive floats += v in one request (dst 16-byte aligned)
+__device__ __forceinline__ void red_add4(float* dst, const float4& v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
 }
 
 // ------------------------------------------------------------------------------------------------
 // RMSNorm forward: optionally res_out = x + delta first.  One warp per row, H % 8 == 0.
 // ------------------------------------------------------------------------------------------------
+template <typename W>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                   NormScale w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
+                   const W* __restrict__ w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
                    float* __restrict__ rstd_out, int rows, int H, float eps) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -104,7 +104,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     for (int v = lane; v < nvec; v += 32) {
       float f[8], wv[8];
       unpack8(src[v], f);
-      load8w(w, v * 8, wv);
+      load8w(w + v * 8, wv);
 #pragma unroll
       for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * wv[i];
       yr[v] = pack8(f);
@@ -114,10 +114,10 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 
 // H == NV * 256: a warp keeps its whole row in registers, so every load of the row is in flight at once and the row
 // is read from memory exactly once (the generic kernel above walks the row twice with one load in flight per lane).
-template <int NV>
+template <int NV, typename W>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                       NormScale w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
+                       const W* __restrict__ w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
                        float* __restrict__ rstd_out, int rows, float eps) {
   constexpr int H = NV * 256;
   const int lane = threadIdx.x & 31;
@@ -158,7 +158,7 @@ rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
     for (int j = 0; j < NV; ++j) {
       float f[8], wv[8];
       unpack8(raw[j], f);
-      load8w(w, (lane + 32 * j) * 8, wv);
+      load8w(w + (lane + 32 * j) * 8, wv);
 #pragma unroll
       for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * wv[i];
       yr[lane + 32 * j] = pack8(f);
@@ -168,9 +168,10 @@ rmsnorm_fwd_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
 
 // The same for a handful of rows (a decode step): one block per row, so that a row's loads are issued by 256 threads at
 // once instead of one warp walking it.
+template <typename W>
 __global__ void __launch_bounds__(256)
 rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                       NormScale w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
+                       const W* __restrict__ w, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y,
                        float* __restrict__ rstd_out, int H, float eps) {
   __shared__ float part[8];
   b200::pdl_launch_dependents();   // no-ops unless launched as a dependent (decode steps)
@@ -209,7 +210,7 @@ rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
   for (int v = threadIdx.x; v < nvec; v += 256) {  // a thread re-reads only what it wrote itself
     float f[8], wv[8];
     unpack8(src[v], f);
-    load8w(w, v * 8, wv);
+    load8w(w + v * 8, wv);
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * wv[i];
     yr[v] = pack8(f);
@@ -235,25 +236,16 @@ splitk_finish_kernel(float* __restrict__ ws, __nv_bfloat16* __restrict__ out, lo
 }
 
 // RMSNorm backward.  dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres if given); dw += sum_rows dy*xhat
-// NV > 0: H == NV * 256 and every lane keeps its dw partial sums in registers over all of its rows;
-// NV == 0: any H % 8 == 0, partial sums go through shared-memory atomics.  Either way a block folds its
-// partials in shared memory and issues one fp32 atomicAdd per column.
-template <int NV>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, (NV == 8 ? 2 : 1))
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, NormScale w,
-                   const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dy,
-                   const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
-                   int rows, int H) {
+// Any H % 8 == 0: one warp per row, the dw partial sums of a block go through shared-memory atomics.
+template <typename W>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ w, const float* __restrict__ rstd_in,
+                   const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres,
+                   __nv_bfloat16* __restrict__ dx, float* __restrict__ dw, int rows, int H) {
   extern __shared__ float dw_smem[];  // H floats
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int nvec = H >> 3;
-  constexpr int NACC = NV > 0 ? NV : 1;
-  float acc[NACC][8];
-#pragma unroll
-  for (int j = 0; j < NACC; ++j)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
   for (int i = threadIdx.x; i < H; i += blockDim.x) dw_smem[i] = 0.f;
   __syncthreads();
   for (long long row = (long long)blockIdx.x * kWarpsPerBlock + warp; row < rows;
@@ -262,92 +254,32 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, NormScale w,
     const uint4* gr = reinterpret_cast<const uint4*>(dy + row * H);
     const float rstd = rstd_in[row];
     float dot = 0.f;
-    // Up to H = 1024 the row of x and dy stays in registers (read once, all loads in flight: 0.61 of the copy
-    // bandwidth against 0.45).  Above that the registers go to the dw partial sums; batching the loads of the first
-    // pass there cost occupancy and measured slower (0.43 against 0.55 at H = 2048).
-    constexpr bool kInRegs = NV > 0 && NV <= 4;
-    constexpr int NRAW = kInRegs ? NV : 1;
-    uint4 xraw[NRAW], graw[NRAW];
-    if constexpr (kInRegs) {
+    for (int v = lane; v < nvec; v += 32) {
+      float f[8], g[8], wv[8];
+      unpack8(xr[v], f);
+      unpack8(gr[v], g);
+      load8w(w + v * 8, wv);
 #pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        xraw[j] = xr[lane + 32 * j];
-        graw[j] = gr[lane + 32 * j];
-      }
-#pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        float f[8], g[8], wv[8];
-        unpack8(xraw[j], f);
-        unpack8(graw[j], g);
-        load8w(w, (lane + 32 * j) * 8, wv);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) dot += g[i] * wv[i] * f[i] * rstd;
-      }
-    } else if constexpr (NV == 8) {
-#pragma unroll 4
-      for (int j = 0; j < NV; ++j) {  // known trip count: four loads of x and of dy in flight per lane
-        const int v = lane + 32 * j;
-        float f[8], g[8], wv[8];
-        unpack8(xr[v], f);
-        unpack8(gr[v], g);
-        load8w(w, v * 8, wv);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) dot += g[i] * wv[i] * f[i] * rstd;
-      }
-    } else {
-      for (int v = lane; v < nvec; v += 32) {
-        float f[8], g[8], wv[8];
-        unpack8(xr[v], f);
-        unpack8(gr[v], g);
-        load8w(w, v * 8, wv);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) dot += g[i] * wv[i] * f[i] * rstd;
-      }
+      for (int i = 0; i < 8; ++i) dot += g[i] * wv[i] * f[i] * rstd;
     }
     dot = warp_sum(dot) / (float)H;
     const uint4* rr = dres ? reinterpret_cast<const uint4*>(dres + row * H) : nullptr;
     uint4* dxr = reinterpret_cast<uint4*>(dx + row * H);
-    if constexpr (NV > 0) {
+    for (int v = lane; v < nvec; v += 32) {
+      float f[8], g[8], wv[8], o[8];
+      unpack8(xr[v], f);
+      unpack8(gr[v], g);
+      load8w(w + v * 8, wv);
+      float r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (rr) unpack8(rr[v], r);
 #pragma unroll
-      for (int j = 0; j < NV; ++j) {
-        const int v = lane + 32 * j;
-        float f[8], g[8], wv[8], o[8];
-        unpack8(kInRegs ? xraw[j < NRAW ? j : 0] : xr[v], f);
-        unpack8(kInRegs ? graw[j < NRAW ? j : 0] : gr[v], g);
-        load8w(w, v * 8, wv);
-        float r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (rr) unpack8(rr[v], r);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float xhat = f[i] * rstd;
-          o[i] = rstd * (g[i] * wv[i] - xhat * dot) + r[i];
-          acc[j][i] += g[i] * xhat;
-        }
-        dxr[v] = pack8(o);
+      for (int i = 0; i < 8; ++i) {
+        const float xhat = f[i] * rstd;
+        o[i] = rstd * (g[i] * wv[i] - xhat * dot) + r[i];
+        atomicAdd(&dw_smem[v * 8 + i], g[i] * xhat);
       }
-    } else {
-      for (int v = lane; v < nvec; v += 32) {
-        float f[8], g[8], wv[8], o[8];
-        unpack8(xr[v], f);
-        unpack8(gr[v], g);
-        load8w(w, v * 8, wv);
-        float r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (rr) unpack8(rr[v], r);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float xhat = f[i] * rstd;
-          o[i] = rstd * (g[i] * wv[i] - xhat * dot) + r[i];
-          atomicAdd(&dw_smem[v * 8 + i], g[i] * xhat);
-        }
-        dxr[v] = pack8(o);
-      }
+      dxr[v] = pack8(o);
     }
-  }
-  if constexpr (NV > 0) {
-#pragma unroll
-    for (int j = 0; j < NV; ++j)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) atomicAdd(&dw_smem[(lane + 32 * j) * 8 + i], acc[j][i]);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < H; i += blockDim.x) {
@@ -356,98 +288,117 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, NormScale w,
   }
 }
 
-// RMSNorm backward for wide rows (H = 8 * VEC * THREADS): a block walks rows, a thread owns 8 * VEC columns of every
-// row, so the row of x and dy is read once into registers, the dw partial sums are 8 * VEC registers, and the loads
-// of the block's next row are issued before the current row is reduced (one block-wide reduction of the dot product
-// through shared memory per row, double buffered by parity), which keeps loads in flight all the time.
-template <int VEC, int THREADS, int MINB>
-__global__ void __launch_bounds__(THREADS, MINB)
-rmsnorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ x, NormScale w,
-                        const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dy,
-                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                        float* __restrict__ dw, int rows, int H) {
-  __shared__ float red[2][32];
+// RMSNorm backward for H = 8 * blockDim.x * VEC: a block walks groups of ROWS rows, a thread owns 8 * VEC columns of
+// them, so x, dy and dres are read once, all 3 * ROWS * VEC 16-byte loads of a group are in flight at once, the dw
+// partial sums are registers, and one block-wide reduction serves ROWS dot products.  What bounds it: memory traffic
+// (three reads and one write of the rows); blocks of at most 256 threads leave room for several per SM, whose loads
+// cover each other's reductions.  One warp per row, which re-reads x and dy for its second pass, took 150 us at 32768
+// rows of 2048 and 294 us at 20000 rows of 3072 where this takes 107 us and 110 us (5.0 and 4.5 TB/s).
+// AHEAD: the next group's loads are issued before the current one is reduced, for rows so wide that one block fills
+// an SM (8000 rows of 8192: 109 us with, 122 us without).
+template <int VEC, int ROWS, int MAXT, int MINB, bool AHEAD, typename W>
+__global__ void __launch_bounds__(MAXT, MINB)
+rmsnorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ w, const float* __restrict__ rstd_in,
+                        const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres,
+                        __nv_bfloat16* __restrict__ dx, float* __restrict__ dw, int rows, int H) {
+  extern __shared__ float dw_smem[];  // H floats
+  __shared__ float red[2][ROWS][32];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  constexpr int kWarps = THREADS / 32;
+  const int warps = blockDim.x >> 5, threads = blockDim.x;
   const long long nvec = H >> 3;
   const float inv_h = 1.f / (float)H;
   float wv[VEC][8], acc[VEC][8];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
-    load8w(w, (t + v * THREADS) * 8, wv[v]);
+    load8w(w + (t + v * threads) * 8, wv[v]);
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
   }
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  uint4 xc[VEC], gc[VEC], rc[VEC];
-  float rs = 0.f;
-  long long row = blockIdx.x;
-  if (row < rows) {
+  uint4 xc[ROWS][VEC], gc[ROWS][VEC], rc[ROWS][VEC];
+  float rs[ROWS];
+  auto load = [&](long long row0, uint4 (&xl)[ROWS][VEC], uint4 (&gl)[ROWS][VEC], uint4 (&rl)[ROWS][VEC],
+                  float (&rsl)[ROWS]) {
+    const uint4 zero = make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) {
-      xc[v] = reinterpret_cast<const uint4*>(x)[row * nvec + t + v * THREADS];
-      gc[v] = reinterpret_cast<const uint4*>(dy)[row * nvec + t + v * THREADS];
-      rc[v] = dres ? reinterpret_cast<const uint4*>(dres)[row * nvec + t + v * THREADS] : zero;
-    }
-    rs = rstd_in[row];
-  }
-  int parity = 0;
-  for (; row < rows; row += gridDim.x, parity ^= 1) {
-    uint4 xn[VEC], gn[VEC], rn[VEC];
-    float rsn = 0.f;
-    const long long next = row + gridDim.x;
-    if (next < rows) {  // in flight while this row is reduced and written
+    for (int r = 0; r < ROWS; ++r) {
+      const long long row = row0 + r;
+      const bool in = row < rows;
 #pragma unroll
       for (int v = 0; v < VEC; ++v) {
-        xn[v] = reinterpret_cast<const uint4*>(x)[next * nvec + t + v * THREADS];
-        gn[v] = reinterpret_cast<const uint4*>(dy)[next * nvec + t + v * THREADS];
-        rn[v] = dres ? reinterpret_cast<const uint4*>(dres)[next * nvec + t + v * THREADS] : zero;
+        const long long at = row * nvec + t + v * threads;
+        xl[r][v] = in ? reinterpret_cast<const uint4*>(x)[at] : zero;
+        gl[r][v] = in ? reinterpret_cast<const uint4*>(dy)[at] : zero;
+        rl[r][v] = in && dres ? reinterpret_cast<const uint4*>(dres)[at] : zero;
       }
-      rsn = rstd_in[next];
-    } else {
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) xn[v] = gn[v] = rn[v] = zero;
+      rsl[r] = in ? rstd_in[row] : 0.f;
     }
-    float d = 0.f;
+  };
+  const long long step = (long long)gridDim.x * ROWS;
+  int parity = 0;
+  if constexpr (AHEAD) load((long long)blockIdx.x * ROWS, xc, gc, rc, rs);
+  for (long long row0 = (long long)blockIdx.x * ROWS; row0 < rows; row0 += step, parity ^= 1) {
+    uint4 xn[ROWS][VEC], gn[ROWS][VEC], rn[ROWS][VEC];
+    float rsn[ROWS];
+    if constexpr (AHEAD)
+      load(row0 + step, xn, gn, rn, rsn);
+    else
+      load(row0, xc, gc, rc, rs);
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) {
-      float f[8], g[8];
-      unpack8(xc[v], f);
-      unpack8(gc[v], g);
+    for (int r = 0; r < ROWS; ++r) {
+      float d = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) d += g[i] * wv[v][i] * f[i];
+      for (int v = 0; v < VEC; ++v) {
+        float f[8], g[8];
+        unpack8(xc[r][v], f);
+        unpack8(gc[r][v], g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d += g[i] * wv[v][i] * f[i];
+      }
+      d = warp_sum(d * rs[r]);
+      if (lane == 0) red[parity][r][warp] = d;
     }
-    d = warp_sum(d * rs);
-    if (lane == 0) red[parity][warp] = d;
     __syncthreads();
-    const float dot = warp_sum(lane < kWarps ? red[parity][lane] : 0.f) * inv_h;
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) {
-      float f[8], g[8], r[8], o[8];
-      unpack8(xc[v], f);
-      unpack8(gc[v], g);
-      unpack8(rc[v], r);
+    for (int r = 0; r < ROWS; ++r) {
+      const float dot = warp_sum(lane < warps ? red[parity][r][lane] : 0.f) * inv_h;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float xhat = f[i] * rs;
-        o[i] = rs * (g[i] * wv[v][i] - xhat * dot) + r[i];
-        acc[v][i] += g[i] * xhat;
+      for (int v = 0; v < VEC; ++v) {
+        float f[8], g[8], b[8], o[8];
+        unpack8(xc[r][v], f);
+        unpack8(gc[r][v], g);
+        unpack8(rc[r][v], b);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float xhat = f[i] * rs[r];
+          o[i] = rs[r] * (g[i] * wv[v][i] - xhat * dot) + b[i];
+          acc[v][i] += g[i] * xhat;
+        }
+        if (row0 + r < rows) reinterpret_cast<uint4*>(dx)[(row0 + r) * nvec + t + v * threads] = pack8(o);
       }
-      reinterpret_cast<uint4*>(dx)[row * nvec + t + v * THREADS] = pack8(o);
     }
+    if constexpr (AHEAD) {
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) {
-      xc[v] = xn[v];
-      gc[v] = gn[v];
-      rc[v] = rn[v];
+      for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+          xc[r][v] = xn[r][v];
+          gc[r][v] = gn[r][v];
+          rc[r][v] = rn[r][v];
+        }
+        rs[r] = rsn[r];
+      }
     }
-    rs = rsn;
   }
+  // dw: columns in order through shared memory, so that a warp's request covers 512 contiguous bytes (a thread's own
+  // eight columns at a time touched 32 sectors a request, and same-sector adds of hundreds of blocks queue up)
 #pragma unroll
   for (int v = 0; v < VEC; ++v)
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (acc[v][i] != 0.f) atomicAdd(&dw[(t + v * THREADS) * 8 + i], acc[v][i]);
+    for (int i = 0; i < 2; ++i)
+      reinterpret_cast<float4*>(dw_smem)[(t + v * threads) * 2 + i] =
+          make_float4(acc[v][4 * i], acc[v][4 * i + 1], acc[v][4 * i + 2], acc[v][4 * i + 3]);
+  __syncthreads();
+  for (int i = t; i < (H >> 2); i += threads) red_add4(dw + 4 * i, reinterpret_cast<const float4*>(dw_smem)[i]);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -465,142 +416,231 @@ __device__ __forceinline__ void sincos_reduced(float x, float* s, float* c) {
   __sincosf(x, s, c);
 }
 
-// A head of D <= 256 elements is handled by `lph` lanes (a power of two, 8 elements per lane), so a warp works on
-// 32 / lph heads at once; reductions stay inside the lane group.
-__device__ __forceinline__ float group_sum(float v, int lph) {
-  for (int off = lph >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+// A head of D <= 256 elements is handled by LPH lanes (a power of two, 8 elements per lane), so a warp works on
+// HPW = 32 / LPH heads at once; reductions stay inside the lane group.
+//
+// A block works on query heads or on key heads only, so one norm scale and one scale gradient live in registers; the
+// first `blocks_first` blocks take the query heads.  A warp takes one token (or, when there are too few tokens to fill
+// the device, a chunk of a token's heads) and walks its heads HPW at a time.  The angles of a token are the same for
+// all of its heads: sine and cosine are computed once per token and lane.  The loads of BATCH groups of heads are
+// issued before the first is used.  What bounds it: memory latency and traffic (one read and one write of the q and k
+// columns forward, two reads and one write backward).  One warp per (token, two heads), with the angles and a 64-bit
+// division for every head, was bound by instruction issue: 32768 tokens of 16 + 8 heads of 128 took 144 us forward and
+// 390 us backward where this takes 87 us and 129 us (4.6 TB/s).
+// Blocks per SM: 2 forward loads a lane and 64 registers beat 4 loads (88 us) and 80 or 48 registers (111 us at 48, which
+// spills); backward 4 pairs of loads and 128 registers beat 2 pairs (139 us) and 80 registers (211 us, spills).
+constexpr int kQkFwdBlocks = 4, kQkBwdBlocks = 2;
+
+template <int LPH>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+  for (int off = LPH >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   return v;
 }
 
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride, __nv_bfloat16* __restrict__ out,
-                       long long out_stride, NormScale w, const int* __restrict__ positions,
-                       float* __restrict__ rstd_out, long long tokens, int heads, int D, float eps, float log2_theta,
-                       int rope, int lph, NormScale w2, int heads_first) {
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int hpw = 32 / lph;
-  const int sub = lane / lph, l = lane % lph;
-  const long long total = tokens * heads;
-  const bool has_cols = l * 8 < D;
-  // heads [0, heads_first) are scaled by w, the rest by w2 (query heads and key heads of a packed projection)
-  float inv_freq[4], wv[8] = {1, 1, 1, 1, 1, 1, 1, 1}, wv2[8] = {1, 1, 1, 1, 1, 1, 1, 1};
+struct QkShape {
+  long long tokens;
+  int heads, heads_first, D;  // heads [0, heads_first) take the first norm scale, the rest the second
+  int blocks_first;           // blocks that work on the first kind of heads
+  int per_chunk;              // groups of HPW heads that a warp takes of a token
+  float log2_theta;
+  int rope;
+};
+
+// What one block walks: heads [h0, h1) of all tokens, dealt to the warps of blocks `block` of `blocks`.
+template <int LPH>
+struct QkWalk {
+  int h0, h1, units, chunks;
+  long long item, items, step;
+  __device__ __forceinline__ QkWalk(const QkShape& q, bool first) {
+    constexpr int HPW = 32 / LPH;
+    h0 = first ? 0 : q.heads_first;
+    h1 = first ? q.heads_first : q.heads;
+    units = (h1 - h0 + HPW - 1) / HPW;
+    chunks = (units + q.per_chunk - 1) / q.per_chunk;
+    items = q.tokens * chunks;
+    const int block = first ? blockIdx.x : blockIdx.x - q.blocks_first;
+    const int blocks = first ? q.blocks_first : gridDim.x - q.blocks_first;
+    item = (long long)block * kWarpsPerBlock + (threadIdx.x >> 5);
+    step = (long long)blocks * kWarpsPerBlock;
+  }
+  __device__ __forceinline__ long long at(const QkShape& q, int& u0, int& u1) const {
+    if (chunks == 1) {
+      u0 = 0;
+      u1 = units;
+      return item;
+    }
+    const long long t = item / chunks;
+    u0 = (int)(item - t * chunks) * q.per_chunk;
+    u1 = min(u0 + q.per_chunk, units);
+    return t;
+  }
+};
+
+__device__ __forceinline__ void qk_angles(const QkShape& q, const int* positions, long long t,
+                                          const float (&inv_freq)[4], float (&sn)[4], float (&cs)[4]) {
+  const float pos = (float)positions[t];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) inv_freq[i] = exp2f(-log2_theta * (2.f * (float)(l * 4 + i)) / (float)D);
+  for (int i = 0; i < 4; ++i) sincos_reduced(pos * inv_freq[i], &sn[i], &cs[i]);
+}
+
+template <int LPH, typename W>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, kQkFwdBlocks)
+qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride, __nv_bfloat16* __restrict__ out,
+                       long long out_stride, const W* __restrict__ w_first, const W* __restrict__ w_rest,
+                       const int* __restrict__ positions, float* __restrict__ rstd_out, const QkShape q, float eps) {
+  constexpr int HPW = 32 / LPH, BATCH = 2;
+  const int lane = threadIdx.x & 31;
+  const int sub = lane / LPH, l = lane % LPH;
+  const bool has_cols = l * 8 < q.D;
+  const bool first = (int)blockIdx.x < q.blocks_first;
+  const W* w = first ? w_first : w_rest;
+  const bool norm = w != nullptr;
+  float inv_freq[4], wv[8] = {1, 1, 1, 1, 1, 1, 1, 1};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) inv_freq[i] = exp2f(-q.log2_theta * (2.f * (float)(l * 4 + i)) / (float)q.D);
   // the norm scales are weights (no predecessor writes them): they are read before the wait for the predecessor
-  if (w && has_cols) load8w(w, l * 8, wv);
-  if (w2 && has_cols) load8w(w2, l * 8, wv2);
+  if (norm && has_cols) load8w(w + l * 8, wv);
   b200::pdl_launch_dependents();   // no-ops unless launched as a dependent (decode steps)
   b200::pdl_wait();
-  const long long groups = (total + hpw - 1) / hpw;
-  for (long long gidx = (long long)blockIdx.x * kWarpsPerBlock + warp; gidx < groups;
-       gidx += (long long)gridDim.x * kWarpsPerBlock) {
-    const long long idx = gidx * hpw + sub;
-    const bool active = has_cols && idx < total;
-    const long long t = idx / heads;
-    const int h = (int)(idx - t * heads);
-    float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (active) unpack8(*reinterpret_cast<const uint4*>(in + t * in_stride + (long long)h * D + l * 8), f);
-    if (w) {
-      float ss = 0.f;
+  for (QkWalk<LPH> k(q, first); k.item < k.items; k.item += k.step) {
+    int u0, u1;
+    const long long t = k.at(q, u0, u1);
+    float sn[4] = {0, 0, 0, 0}, cs[4] = {1, 1, 1, 1};
+    if (q.rope) qk_angles(q, positions, t, inv_freq, sn, cs);
+    const __nv_bfloat16* src = in + t * in_stride + l * 8;
+    __nv_bfloat16* dst = out + t * out_stride + l * 8;
+#pragma unroll 1
+    for (int u = u0; u < u1; u += BATCH) {
+      uint4 raw[BATCH];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) ss += f[i] * f[i];
-      ss = group_sum(ss, lph);
-      const float rstd = rsqrtf(ss / (float)D + eps);
-      if (l == 0 && rstd_out && idx < total) rstd_out[idx] = rstd;
-      const bool first = h < heads_first;
+      for (int j = 0; j < BATCH; ++j) {
+        const int h = k.h0 + (u + j) * HPW + sub;
+        raw[j] = make_uint4(0, 0, 0, 0);
+        if (u + j < u1 && has_cols && h < k.h1) raw[j] = *reinterpret_cast<const uint4*>(src + h * q.D);
+      }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * (first ? wv[i] : wv2[i]);
-    }
-    if (rope && active) {
-      const float pos = (float)positions[t];
+      for (int j = 0; j < BATCH; ++j) {
+        if (u + j >= u1) break;
+        const int h = k.h0 + (u + j) * HPW + sub;
+        float f[8];
+        unpack8(raw[j], f);
+        if (norm) {
+          float ss = 0.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float s, c;
-        sincos_reduced(pos * inv_freq[i], &s, &c);
-        const float a = f[2 * i], b = f[2 * i + 1];
-        f[2 * i] = a * c - b * s;
-        f[2 * i + 1] = a * s + b * c;
+          for (int i = 0; i < 8; ++i) ss += f[i] * f[i];
+          ss = group_sum<LPH>(ss);
+          const float rstd = rsqrtf(ss / (float)q.D + eps);
+          if (l == 0 && rstd_out && h < k.h1) rstd_out[t * q.heads + h] = rstd;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * wv[i];
+        }
+        if (q.rope) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float x = f[2 * i], y = f[2 * i + 1];
+            f[2 * i] = x * cs[i] - y * sn[i];
+            f[2 * i + 1] = x * sn[i] + y * cs[i];
+          }
+        }
+        if (has_cols && h < k.h1) *reinterpret_cast<uint4*>(dst + h * q.D) = pack8(f);
       }
     }
-    if (active) *reinterpret_cast<uint4*>(out + t * out_stride + (long long)h * D + l * 8) = pack8(f);
   }
 }
 
-// backward of the above: grad wrt the pre-norm input, and dw (atomic fp32 adds, D columns)
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride,
-                       const __nv_bfloat16* __restrict__ dout, long long dout_stride,
-                       __nv_bfloat16* __restrict__ din, long long din_stride, NormScale w,
-                       const int* __restrict__ positions, const float* __restrict__ rstd_in,
-                       float* __restrict__ dw, long long tokens, int heads, int D, float log2_theta, int rope,
-                       int lph, NormScale w2, float* __restrict__ dw2, int heads_first) {
-  __shared__ float dw_smem[512];
+// backward of the above: gradient of the pre-norm input, and of the scales (atomic fp32 adds, D columns).  `dout` and
+// `din` may be the same buffer: a lane reads its elements of a head before it writes them, and no other lane does.
+template <int LPH, typename W>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, kQkBwdBlocks)
+qknorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride, const __nv_bfloat16* dout,
+                       long long dout_stride, __nv_bfloat16* din, long long din_stride,
+                       const W* __restrict__ w_first, const W* __restrict__ w_rest, const int* __restrict__ positions,
+                       const float* __restrict__ rstd_in, float* __restrict__ dw_first, float* __restrict__ dw_rest,
+                       const QkShape q) {
+  constexpr int HPW = 32 / LPH, BATCH = 4;
+  __shared__ float dw_smem[256];
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int hpw = 32 / lph;
-  const int sub = lane / lph, l = lane % lph;
-  const long long total = tokens * heads;
-  const bool has_cols = l * 8 < D;
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) dw_smem[i] = 0.f;
+  const int sub = lane / LPH, l = lane % LPH;
+  const bool has_cols = l * 8 < q.D;
+  const bool first = (int)blockIdx.x < q.blocks_first;
+  const W* w = first ? w_first : w_rest;
+  float* dw = first ? dw_first : dw_rest;
+  const bool norm = w != nullptr;
+  dw_smem[threadIdx.x] = 0.f;
   __syncthreads();
-  float inv_freq[4], wv[8] = {0, 0, 0, 0, 0, 0, 0, 0}, wv2[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  float inv_freq[4], wv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-  for (int i = 0; i < 4; ++i) inv_freq[i] = exp2f(-log2_theta * (2.f * (float)(l * 4 + i)) / (float)D);
-  if (w && has_cols) load8w(w, l * 8, wv);
-  if (w2 && has_cols) load8w(w2, l * 8, wv2);
-  float dw_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, dw_acc2[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  const long long groups = (total + hpw - 1) / hpw;
-  for (long long gidx = (long long)blockIdx.x * kWarpsPerBlock + warp; gidx < groups;
-       gidx += (long long)gridDim.x * kWarpsPerBlock) {
-    const long long idx = gidx * hpw + sub;
-    const bool active = has_cols && idx < total;
-    const long long t = idx / heads;
-    const int h = (int)(idx - t * heads);
-    float g[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (active) unpack8(*reinterpret_cast<const uint4*>(dout + t * dout_stride + (long long)h * D + l * 8), g);
-    if (rope && active) {
-      const float pos = (float)positions[t];
+  for (int i = 0; i < 4; ++i) inv_freq[i] = exp2f(-q.log2_theta * (2.f * (float)(l * 4 + i)) / (float)q.D);
+  if (norm && has_cols) load8w(w + l * 8, wv);
+  const float inv_d = 1.f / (float)q.D;
+  float dw_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (QkWalk<LPH> k(q, first); k.item < k.items; k.item += k.step) {
+    int u0, u1;
+    const long long t = k.at(q, u0, u1);
+    float sn[4] = {0, 0, 0, 0}, cs[4] = {1, 1, 1, 1};
+    if (q.rope) qk_angles(q, positions, t, inv_freq, sn, cs);
+    const __nv_bfloat16* xsrc = in + t * in_stride + l * 8;
+    const __nv_bfloat16* gsrc = dout + t * dout_stride + l * 8;
+    __nv_bfloat16* dst = din + t * din_stride + l * 8;
+    const float* rstds = rstd_in + t * q.heads;
+#pragma unroll 1
+    for (int u = u0; u < u1; u += BATCH) {
+      uint4 graw[BATCH], xraw[BATCH];
+      float rstd[BATCH];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float s, c;
-        sincos_reduced(pos * inv_freq[i], &s, &c);
-        const float a = g[2 * i], b = g[2 * i + 1];  // transpose of the rotation
-        g[2 * i] = a * c + b * s;
-        g[2 * i + 1] = -a * s + b * c;
+      for (int j = 0; j < BATCH; ++j) {
+        const int h = k.h0 + (u + j) * HPW + sub;
+        const bool valid = u + j < u1 && h < k.h1;
+        graw[j] = xraw[j] = make_uint4(0, 0, 0, 0);
+        rstd[j] = 0.f;
+        if (valid && has_cols) graw[j] = *reinterpret_cast<const uint4*>(gsrc + h * q.D);
+        if (norm && valid) {
+          if (has_cols) xraw[j] = *reinterpret_cast<const uint4*>(xsrc + h * q.D);
+          rstd[j] = rstds[h];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < BATCH; ++j) {
+        if (u + j >= u1) break;
+        const int h = k.h0 + (u + j) * HPW + sub;
+        float g[8];
+        unpack8(graw[j], g);
+        if (q.rope) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float x = g[2 * i], y = g[2 * i + 1];  // transpose of the rotation
+            g[2 * i] = x * cs[i] + y * sn[i];
+            g[2 * i + 1] = -x * sn[i] + y * cs[i];
+          }
+        }
+        if (norm) {
+          float f[8];
+          unpack8(xraw[j], f);
+          float dot = 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            f[i] *= rstd[j];
+            dot += g[i] * wv[i] * f[i];
+          }
+          dot = group_sum<LPH>(dot) * inv_d;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            dw_acc[i] += g[i] * f[i];
+            g[i] = rstd[j] * (g[i] * wv[i] - f[i] * dot);
+          }
+        }
+        if (has_cols && h < k.h1) *reinterpret_cast<uint4*>(dst + h * q.D) = pack8(g);
       }
     }
-    if (w) {
-      float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (active) unpack8(*reinterpret_cast<const uint4*>(in + t * in_stride + (long long)h * D + l * 8), f);
-      const float rstd = idx < total ? rstd_in[idx] : 0.f;
-      const bool first = h < heads_first;
-      float dot = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) dot += g[i] * (first ? wv[i] : wv2[i]) * f[i] * rstd;
-      dot = group_sum(dot, lph) / (float)D;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float xhat = f[i] * rstd;
-        if (first) dw_acc[i] += g[i] * xhat; else dw_acc2[i] += g[i] * xhat;
-        g[i] = rstd * (g[i] * (first ? wv[i] : wv2[i]) - xhat * dot);
-      }
-    }
-    if (active) *reinterpret_cast<uint4*>(din + t * din_stride + (long long)h * D + l * 8) = pack8(g);
   }
-  if (w && (dw || dw2)) {
+  if (norm && dw) {
     if (has_cols) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        atomicAdd(&dw_smem[l * 8 + i], dw_acc[i]);
-        atomicAdd(&dw_smem[256 + l * 8 + i], dw_acc2[i]);
-      }
+      for (int i = 0; i < 8; ++i) atomicAdd(&dw_smem[l * 8 + i], dw_acc[i]);
     }
     __syncthreads();
-    if (threadIdx.x < D) {
-      if (dw) atomicAdd(&dw[threadIdx.x], dw_smem[threadIdx.x]);
-      if (dw2) atomicAdd(&dw2[threadIdx.x], dw_smem[256 + threadIdx.x]);
-    }
+    if (threadIdx.x < q.D) atomicAdd(&dw[threadIdx.x], dw_smem[threadIdx.x]);
   }
 }
 
@@ -1062,21 +1102,21 @@ inline int grid_for(long long work_items, int block, int per_sm = 8) {
 #define STREAM(s) reinterpret_cast<cudaStream_t>(s)
 #define LAST_ERR() static_cast<int>(cudaGetLastError())
 
-extern "C" int b200_rmsnorm_fwd(const void* x, const void* delta, const void* w, int w_bf16, void* res_out, void* y, void* rstd,
-                                int rows, int H, float eps, void* stream) {
-  if (H % 8) return -2;
+template <typename W>
+static int rmsnorm_fwd_launch(const void* x, const void* delta, const W* w, void* res_out, void* y, void* rstd, int rows,
+                              int H, float eps, void* stream) {
   if (rows > 0 && rows <= 512) {
     // few rows = a decode step: launched as a dependent so that it is resident when its predecessor ends
     return static_cast<int>(b200host::launch_kernel(
-        rmsnorm_fwd_row_kernel, dim3(rows), dim3(256), 0, STREAM(stream), b200host::pdl_enabled() != 0,
-        (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, NormScale{w, w_bf16}, (__nv_bfloat16*)res_out,
-        (__nv_bfloat16*)y, (float*)rstd, H, eps));
+        rmsnorm_fwd_row_kernel<W>, dim3(rows), dim3(256), 0, STREAM(stream), b200host::pdl_enabled() != 0,
+        (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, w, (__nv_bfloat16*)res_out, (__nv_bfloat16*)y,
+        (float*)rstd, H, eps));
   }
   const int grid = grid_for((long long)rows, kWarpsPerBlock, 8);
 #define RMS_FWD(NV)                                                                                         \
-  rmsnorm_fwd_reg_kernel<NV><<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(                             \
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, NormScale{w, w_bf16}, (__nv_bfloat16*)res_out,       \
-      (__nv_bfloat16*)y, (float*)rstd, rows, eps);                                                         \
+  rmsnorm_fwd_reg_kernel<NV, W><<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(                          \
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, w, (__nv_bfloat16*)res_out, (__nv_bfloat16*)y,  \
+      (float*)rstd, rows, eps);                                                                             \
   return LAST_ERR()
   switch (H) {
     case 1024: RMS_FWD(4);
@@ -1085,98 +1125,144 @@ extern "C" int b200_rmsnorm_fwd(const void* x, const void* delta, const void* w,
     default: break;
   }
 #undef RMS_FWD
-  rmsnorm_fwd_kernel<<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, NormScale{w, w_bf16}, (__nv_bfloat16*)res_out,
-      (__nv_bfloat16*)y, (float*)rstd, rows, H, eps);
+  rmsnorm_fwd_kernel<W><<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, w, (__nv_bfloat16*)res_out, (__nv_bfloat16*)y,
+      (float*)rstd, rows, H, eps);
   return LAST_ERR();
 }
-extern "C" int b200_rmsnorm_bwd(const void* x, const void* w, int w_bf16, const void* rstd, const void* dy, const void* dres,
-                                void* dx, void* dw, int rows, int H, void* stream) {
-  if (H % 8 || H * 4 > 48 * 1024) return -2;
-  if (H == 4096 || H == 8192) {   // narrower rows: the warp-per-row kernel below measured faster
-#define RMS_BWD_COLS(VEC, THREADS, MINB)                                                                        \
-  rmsnorm_bwd_cols_kernel<VEC, THREADS, MINB><<<grid_for((long long)rows, 1, MINB), THREADS, 0, STREAM(stream)>>>( \
-      (const __nv_bfloat16*)x, NormScale{w, w_bf16}, (const float*)rstd, (const __nv_bfloat16*)dy,                   \
-      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (float*)dw, rows, H)
-    if (H == 4096) RMS_BWD_COLS(2, 256, 2);
-    else RMS_BWD_COLS(2, 512, 1);
+extern "C" int b200_rmsnorm_fwd(const void* x, const void* delta, const void* w, int w_bf16, void* res_out, void* y,
+                                void* rstd, int rows, int H, float eps, void* stream) {
+  if (H % 8) return -2;
+  if (w_bf16)
+    return rmsnorm_fwd_launch(x, delta, (const __nv_bfloat16*)w, res_out, y, rstd, rows, H, eps, stream);
+  return rmsnorm_fwd_launch(x, delta, (const float*)w, res_out, y, rstd, rows, H, eps, stream);
+}
+template <typename W>
+static int rmsnorm_bwd_launch(const void* x, const W* w, const void* rstd, const void* dy, const void* dres, void* dx,
+                              void* dw, int rows, int H, void* stream) {
+  const bool dw16 = (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
+#define RMS_BWD_COLS(VEC, ROWS, THREADS, MAXT, MINB, AHEAD)                                                           \
+  do {                                                                                                                \
+    rmsnorm_bwd_cols_kernel<VEC, ROWS, MAXT, MINB, AHEAD, W>                                                          \
+        <<<grid_for(((long long)rows + ROWS - 1) / ROWS, 1, MINB * (MAXT / (THREADS))), THREADS, H * sizeof(float),   \
+           STREAM(stream)>>>(                                                                                         \
+            (const __nv_bfloat16*)x, w, (const float*)rstd, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres,     \
+            (__nv_bfloat16*)dx, (float*)dw, rows, H);                                                                 \
+    return LAST_ERR();                                                                                                \
+  } while (0)
+  // whole warps of columns: one 16-byte vector of a row per thread up to 2048 columns, two above
+  if (dw16 && H % 256 == 0 && H <= 512) RMS_BWD_COLS(1, 4, H / 8, 64, 8, false);
+  if (dw16 && H % 256 == 0 && H <= 2048) RMS_BWD_COLS(1, 2, H / 8, 256, 4, false);
+  if (dw16 && H % 512 == 0 && H <= 4096) RMS_BWD_COLS(2, 1, H / 16, 256, 3, false);
+  if (dw16 && H % 512 == 0 && H <= 8192) RMS_BWD_COLS(2, 1, H / 16, 512, 1, true);
 #undef RMS_BWD_COLS
-    return LAST_ERR();
-  }
   const int grid = grid_for((long long)rows, kWarpsPerBlock, 2);
-#define RMS_BWD(NV)                                                                                     \
-  rmsnorm_bwd_kernel<NV><<<grid, kWarpsPerBlock * 32, H * sizeof(float), STREAM(stream)>>>(              \
-      (const __nv_bfloat16*)x, NormScale{w, w_bf16}, (const float*)rstd, (const __nv_bfloat16*)dy,            \
-      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (float*)dw, rows, H)
-  switch (H) {
-    case 256: RMS_BWD(1); break;
-    case 512: RMS_BWD(2); break;
-    case 1024: RMS_BWD(4); break;
-    case 2048: RMS_BWD(8); break;
-    case 4096: RMS_BWD(16); break;
-    default: RMS_BWD(0); break;
-  }
-#undef RMS_BWD
+  rmsnorm_bwd_kernel<W><<<grid, kWarpsPerBlock * 32, H * sizeof(float), STREAM(stream)>>>(
+      (const __nv_bfloat16*)x, w, (const float*)rstd, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres,
+      (__nv_bfloat16*)dx, (float*)dw, rows, H);
   return LAST_ERR();
+}
+extern "C" int b200_rmsnorm_bwd(const void* x, const void* w, int w_bf16, const void* rstd, const void* dy,
+                                const void* dres, void* dx, void* dw, int rows, int H, void* stream) {
+  if (H % 8 || H * 4 > 48 * 1024) return -2;
+  if (w_bf16)
+    return rmsnorm_bwd_launch(x, (const __nv_bfloat16*)w, rstd, dy, dres, dx, dw, rows, H, stream);
+  return rmsnorm_bwd_launch(x, (const float*)w, rstd, dy, dres, dx, dw, rows, H, stream);
 }
 static int lanes_per_head(int D) {
   int lph = 1;
   while (lph * 8 < D) lph <<= 1;
   return lph;
 }
-extern "C" int b200_qknorm_rope_fwd(const void* in, long long in_stride, void* out, long long out_stride,
-                                    const void* w, int w_bf16, const void* positions, void* rstd, long long tokens, int heads,
-                                    int D, float eps, float theta, int rope, void* stream) {
-  if (D % 8 || D > 256) return -2;
-  const int lph = lanes_per_head(D);
-  const int grid = grid_for((tokens * heads + 32 / lph - 1) / (32 / lph), kWarpsPerBlock, 8);
-  return static_cast<int>(b200host::launch_kernel(qknorm_rope_fwd_kernel, dim3(grid), dim3(kWarpsPerBlock * 32), 0,
-                                                  STREAM(stream), tokens <= 512 && b200host::pdl_enabled() != 0,
-      (const __nv_bfloat16*)in, in_stride, (__nv_bfloat16*)out, out_stride, NormScale{w, w_bf16}, (const int*)positions,
-      (float*)rstd, tokens, heads, D, eps, log2f(theta), rope, lph, NormScale{nullptr, 0}, heads));
+// A warp per token and kind of heads where that gives every scheduler of the device eight warps; with fewer tokens (a
+// decode step, short sequences) a token's heads are dealt to more warps, down to one group of heads each.  The blocks
+// are shared out between query and key heads by their number of groups.
+static int qk_shape(QkShape& q, long long tokens, int heads_first, int heads, int D, float theta, int rope,
+                    int blocks_per_sm) {
+  const int hpw = 32 / lanes_per_head(D);
+  const int first = (heads_first + hpw - 1) / hpw, rest = (heads - heads_first + hpw - 1) / hpw;
+  const int most = first > rest ? first : rest;
+  const long long want = 148 * 32;
+  long long per = tokens >= want ? most : (tokens * (first + rest) + want - 1) / want;
+  per = per < 1 ? 1 : (per > most ? most : per);
+  const long long items_first = tokens * ((first + per - 1) / per), items_rest = tokens * ((rest + per - 1) / per);
+  int grid = grid_for(items_first + items_rest, kWarpsPerBlock, blocks_per_sm);
+  int blocks_first = grid * first / (first + rest);
+  if (first && blocks_first == 0) blocks_first = 1;
+  if (rest && blocks_first >= grid) grid = blocks_first + 1;
+  if (!rest) blocks_first = grid;
+  q = QkShape{tokens, heads, heads_first, D, blocks_first, (int)per, log2f(theta), rope};
+  return grid;
 }
+#define QK_DISPATCH(D, CALL)            \
+  switch (lanes_per_head(D)) {          \
+    case 1: CALL(1);                    \
+    case 2: CALL(2);                    \
+    case 4: CALL(4);                    \
+    case 8: CALL(8);                    \
+    case 16: CALL(16);                  \
+    default: CALL(32);                  \
+  }
 // Query and key heads of a packed projection in one launch: the first heads_q heads use wq, the next heads_k use wk
 // (both or neither given); rstd is [tokens, heads_q + heads_k].
 extern "C" int b200_qknorm_rope_fwd_qk(const void* in, long long in_stride, void* out, long long out_stride,
                                        const void* wq, const void* wk, int w_bf16, const void* positions, void* rstd,
                                        long long tokens, int heads_q, int heads_k, int D, float eps, float theta,
                                        int rope, void* stream) {
-  if (D % 8 || D > 256 || (wq == nullptr) != (wk == nullptr)) return -2;
-  const int heads = heads_q + heads_k;
-  const int lph = lanes_per_head(D);
-  const int grid = grid_for((tokens * heads + 32 / lph - 1) / (32 / lph), kWarpsPerBlock, 8);
-  return static_cast<int>(b200host::launch_kernel(qknorm_rope_fwd_kernel, dim3(grid), dim3(kWarpsPerBlock * 32), 0,
-                                                  STREAM(stream), tokens <= 512 && b200host::pdl_enabled() != 0,
-      (const __nv_bfloat16*)in, in_stride, (__nv_bfloat16*)out, out_stride, NormScale{wq, w_bf16}, (const int*)positions,
-      (float*)rstd, tokens, heads, D, eps, log2f(theta), rope, lph, NormScale{wk, w_bf16}, heads_q));
+  if (D % 8 || D > 256 || (heads_k && (wq == nullptr) != (wk == nullptr))) return -2;
+  if (tokens <= 0 || heads_q + heads_k <= 0) return 0;
+  QkShape q;
+  const int grid = qk_shape(q, tokens, heads_q, heads_q + heads_k, D, theta, rope, kQkFwdBlocks);
+#define QK_FWD_AS(LPH, W)                                                                                             \
+  return static_cast<int>(b200host::launch_kernel(                                                                    \
+      qknorm_rope_fwd_kernel<LPH, W>, dim3(grid), dim3(kWarpsPerBlock * 32), 0, STREAM(stream),                       \
+      tokens <= 512 && b200host::pdl_enabled() != 0, (const __nv_bfloat16*)in, in_stride, (__nv_bfloat16*)out,        \
+      out_stride, (const W*)wq, (const W*)wk, (const int*)positions, (float*)rstd, q, eps))
+#define QK_FWD(LPH)                          \
+  if (w_bf16) QK_FWD_AS(LPH, __nv_bfloat16); \
+  QK_FWD_AS(LPH, float)
+  QK_DISPATCH(D, QK_FWD)
+#undef QK_FWD
+#undef QK_FWD_AS
+}
+extern "C" int b200_qknorm_rope_fwd(const void* in, long long in_stride, void* out, long long out_stride,
+                                    const void* w, int w_bf16, const void* positions, void* rstd, long long tokens,
+                                    int heads, int D, float eps, float theta, int rope, void* stream) {
+  return b200_qknorm_rope_fwd_qk(in, in_stride, out, out_stride, w, nullptr, w_bf16, positions, rstd, tokens, heads, 0,
+                                 D, eps, theta, rope, stream);
+}
+extern "C" int b200_qknorm_rope_bwd_qk(const void* in, long long in_stride, const void* dout, long long dout_stride,
+                                       void* din, long long din_stride, const void* wq, const void* wk, int w_bf16,
+                                       const void* positions, const void* rstd, void* dwq, void* dwk,
+                                       long long tokens, int heads_q, int heads_k, int D, float theta, int rope,
+                                       void* stream) {
+  if (D % 8 || D > 256 || (heads_k && (wq == nullptr) != (wk == nullptr))) return -2;
+  if (tokens <= 0 || heads_q + heads_k <= 0) return 0;
+  QkShape q;
+  const int grid = qk_shape(q, tokens, heads_q, heads_q + heads_k, D, theta, rope, kQkBwdBlocks);
+#define QK_BWD_AS(LPH, W)                                                                                           \
+  {                                                                                                                 \
+    qknorm_rope_bwd_kernel<LPH, W><<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(                               \
+        (const __nv_bfloat16*)in, in_stride, (const __nv_bfloat16*)dout, dout_stride, (__nv_bfloat16*)din,          \
+        din_stride, (const W*)wq, (const W*)wk, (const int*)positions, (const float*)rstd, (float*)dwq,             \
+        (float*)dwk, q);                                                                                            \
+    return LAST_ERR();                                                                                              \
+  }
+#define QK_BWD(LPH)                         \
+  if (w_bf16) QK_BWD_AS(LPH, __nv_bfloat16) \
+  QK_BWD_AS(LPH, float)
+  QK_DISPATCH(D, QK_BWD)
+#undef QK_BWD
+#undef QK_BWD_AS
 }
 extern "C" int b200_qknorm_rope_bwd(const void* in, long long in_stride, const void* dout, long long dout_stride,
                                     void* din, long long din_stride, const void* w, int w_bf16, const void* positions,
                                     const void* rstd, void* dw, long long tokens, int heads, int D, float theta,
                                     int rope, void* stream) {
-  if (D % 8 || D > 256) return -2;
-  const int lph = lanes_per_head(D);
-  const int grid = grid_for((tokens * heads + 32 / lph - 1) / (32 / lph), kWarpsPerBlock, 4);
-  qknorm_rope_bwd_kernel<<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(
-      (const __nv_bfloat16*)in, in_stride, (const __nv_bfloat16*)dout, dout_stride, (__nv_bfloat16*)din, din_stride,
-      NormScale{w, w_bf16}, (const int*)positions, (const float*)rstd, (float*)dw, tokens, heads, D, log2f(theta), rope,
-      lph, NormScale{nullptr, 0}, nullptr, heads);
-  return LAST_ERR();
+  return b200_qknorm_rope_bwd_qk(in, in_stride, dout, dout_stride, din, din_stride, w, nullptr, w_bf16, positions, rstd,
+                                 dw, nullptr, tokens, heads, 0, D, theta, rope, stream);
 }
-extern "C" int b200_qknorm_rope_bwd_qk(const void* in, long long in_stride, const void* dout, long long dout_stride,
-                                       void* din, long long din_stride, const void* wq, const void* wk,
-                                       int w_bf16, const void* positions, const void* rstd, void* dwq, void* dwk, long long tokens,
-                                       int heads_q, int heads_k, int D, float theta, int rope, void* stream) {
-  if (D % 8 || D > 256 || (wq == nullptr) != (wk == nullptr)) return -2;
-  const int heads = heads_q + heads_k;
-  const int lph = lanes_per_head(D);
-  const int grid = grid_for((tokens * heads + 32 / lph - 1) / (32 / lph), kWarpsPerBlock, 4);
-  qknorm_rope_bwd_kernel<<<grid, kWarpsPerBlock * 32, 0, STREAM(stream)>>>(
-      (const __nv_bfloat16*)in, in_stride, (const __nv_bfloat16*)dout, dout_stride, (__nv_bfloat16*)din, din_stride,
-      NormScale{wq, w_bf16}, (const int*)positions, (const float*)rstd, (float*)dwq, tokens, heads, D, log2f(theta), rope,
-      lph, NormScale{wk, w_bf16}, (float*)dwk, heads_q);
-  return LAST_ERR();
-}
+#undef QK_DISPATCH
 extern "C" int b200_swiglu_fwd(const void* gu, void* h, long long rows, int I, void* stream) {
   if (I % 8 || rows * (I / 8) >= (1LL << 32)) return -2;
   return static_cast<int>(b200host::launch_kernel(swiglu_fwd_kernel, dim3(grid_for(rows * (I / 8), 256)), dim3(256), 0,

@@ -63,6 +63,59 @@ def test_norm_scales_are_read_in_the_precision_they_are_held_in(H, rows):
         native.rmsnorm_fwd(x, wb.half(), 1e-6)
 
 
+def _off(got, ref):
+    return float((got.detach().double() - ref.detach().double()).norm() / ref.detach().double().norm())
+
+
+# widths on each side of the kernel's choices of columns per thread, rows around a block's group of rows
+@pytest.mark.parametrize("H", [256, 512, 768, 2048, 2560, 4096, 5632, 8192, 8200])
+@pytest.mark.parametrize("rows", [1, 5, 1203])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_rmsnorm_bwd_widths(H, rows, with_res):
+    from research_b200.ops import native
+
+    x, dy = _bf((rows, H), 31), _bf((rows, H), 32)
+    dres = _bf((rows, H), 33) if with_res else None
+    w = torch.rand(H, device="cuda") + 0.5
+    _, rstd, _ = native.rmsnorm_fwd(x, w, 1e-6)
+    xr, wr = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    (xr * torch.rsqrt(xr.pow(2).mean(-1, keepdim=True) + 1e-6) * wr).backward(dy.double())
+    dw = torch.ones(H, device="cuda")                                   # accumulated into
+    dx = native.rmsnorm_bwd(x, w, rstd, dy, dw, dres)
+    # one rounding to bf16 (2^-9 of each value); fp32 sums of at most 1203 terms (2^-24 each) on top of the 1
+    assert _off(dx, xr.grad + (0 if dres is None else dres.double())) < 2.0 ** -9
+    assert _off(dw, wr.grad + 1) < 1e-5
+
+
+# odd head counts, tokens on both sides of the rule that deals a token's heads to several warps (4736 tokens)
+@pytest.mark.parametrize("T,hq,hkv,D", [(1, 1, 1, 128), (33, 3, 1, 64), (700, 5, 3, 128), (700, 7, 1, 96),
+                                        (4735, 2, 1, 64), (4740, 3, 2, 128), (9, 2, 2, 256), (50, 4, 4, 8)])
+def test_qknorm_rope_shapes(T, hq, hkv, D):
+    from research_b200.ops import native
+
+    buf, dout = _bf((T, (hq + 2 * hkv) * D), 41), _bf((T, (hq + hkv) * D), 42)
+    pos = torch.arange(T, device="cuda", dtype=torch.int32) % 251
+    wq, wk = torch.rand(D, device="cuda") + 0.5, torch.rand(D, device="cuda") + 0.5
+    out = torch.zeros(T, (hq + hkv) * D, dtype=torch.bfloat16, device="cuda")
+    r = native.qknorm_rope_fwd_qk(buf, out, wq, wk, pos, hq, hkv, D, 1e-6, 10000.0, True)
+    x = buf[:, :(hq + hkv) * D].double().view(T, hq + hkv, D).requires_grad_(True)
+    ws = [wq.double().requires_grad_(True), wk.double().requires_grad_(True)]
+    scale = torch.cat([ws[0].expand(hq, D), ws[1].expand(hkv, D)])
+    ref = _rope_ref(x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * scale, pos.double(), 10000.0)
+    grads = torch.autograd.grad([ref], [x] + ws, [dout.double().view(T, hq + hkv, D)])
+    din = torch.zeros_like(buf)
+    dq, dk = torch.zeros(D, device="cuda"), torch.zeros(D, device="cuda")
+    native.qknorm_rope_bwd_qk(buf, dout, din, wq, wk, pos, r, dq, dk, hq, hkv, D, 10000.0, True)
+    same = dout.clone()
+    native.qknorm_rope_bwd_qk(buf, same, same, wq, wk, pos, r, torch.zeros_like(dq), torch.zeros_like(dk), hq, hkv, D,
+                              10000.0, True)
+    # one rounding to bf16; the angle is formed in fp32: 251 * 2^-24 = 1.5e-5
+    assert _off(out.view(T, hq + hkv, D), ref) < 2.0 ** -9
+    assert _off(din[:, :(hq + hkv) * D].view(T, hq + hkv, D), grads[0]) < 2.0 ** -9
+    assert _off(dq, grads[1]) < 1e-4 and _off(dk, grads[2]) < 1e-4
+    assert torch.equal(same, din[:, :(hq + hkv) * D]) and not din[:, (hq + hkv) * D:].any()
+
+
 def _rope_ref(x, pos, theta):
     D = x.shape[-1]
     inv = theta ** (-torch.arange(0, D, 2, device=x.device, dtype=torch.float32) / D)
