@@ -2,12 +2,23 @@
 //
 // One CTA owns 256 query rows of one (batch, head): two 128-row tiles that ping-pong through the
 // tensor core so that the softmax of one tile overlaps the MMAs of the other.
-//   warp 0      TMA producer: both Q tiles once, then K/V blocks of 128 rows through a 3-slot ring
+//   warp 0      TMA producer: both Q tiles once, then K/V blocks of 128 rows through a 5-slot ring
 //   warp 1      MMA issuer  : S_t = Q_t K^T (TMEM, 128 cols per tile), O_t += P_t V (TMEM, D cols)
 //   warps 2-5   softmax of tile 0, warps 6-9 softmax of tile 1: one thread per query row reads its
-//               row of S with tcgen05.ld, keeps the running max / sum, writes P (bf16) into 128-byte
-//               swizzled shared memory for the second MMA, and rescales O in TMEM only when the
-//               running max moved by more than 2^8 (so most blocks skip the rescale).
+//               row of S with tcgen05.ld, keeps the running max / sum, writes P (bf16) over the first
+//               half of S in tensor memory, where the second MMA takes it as its A operand, and rescales
+//               O in TMEM only when the running max moved by more than 2^8 (so most blocks skip the
+//               rescale).
+// What bounds it: a 128 x 128 block of a tile is 2 x 512 clocks of the tensor pipe and 16384 exponentials (1024 clocks of
+// the special-function units), so the two tiles of a CTA have to overlap; the loop of one tile, softmax -> PV -> QK^T ->
+// softmax, takes about 1600 + 1024 + 600 clocks and sets the pace.  The tensor pipe runs its MMAs in the order they are
+// issued: PV(j) of a tile, which reads P, precedes QK^T(j+1), which overwrites it with the next S, and S(j+1) being
+// complete says that PV(j) is, so neither needs a barrier of its own.  The scores are read from tensor memory once, the
+// maximum takes three operands an instruction, the scaling and the sum two lanes, and the loop bounds that select
+// descriptors are made warp-uniform (b200.cuh: warp_uniform).  With P in shared memory, a pass for the maximum and
+// descriptors in ordinary registers the loop took 6100 clocks: 8 x 4096 tokens of 16 / 8 heads of 128, causal, 782 us,
+// now 548 (703 -> 1004 TFLOP/s); 16384 tokens 1382 us, now 898 (1224 TFLOP/s).  A quarter of the exponentials as
+// polynomials on the FMA pipes made it slower (920 us).
 // Masks: every query row attends to kv positions in [lo[row], row] (causal) or [lo[row], S) (not
 // causal); `lo` (int32 [B,S], non-decreasing along S, optional) encodes document starts and sliding
 // windows, and whole kv blocks left of lo[first row] or right of the last row are skipped.
@@ -21,6 +32,8 @@
 // cast to the compute dtype (models/components/attention.py:269-278); masks from
 // models/components/masks.py:9-48.  Its vendored Blackwell comparator (other head dims, no backward, no
 // document mask) is third_party/ThunderKittens/kernels/attention/bf16_b300_mha_causal/bf16_b300_mha_causal.cu.
+#include <type_traits>
+
 #include "b200.cuh"
 #include "host_util.cuh"
 #include "ring.cuh"
@@ -32,17 +45,15 @@ namespace {
 constexpr int NT = 2;          // query tiles per CTA
 constexpr int TILE_M = 128;    // query rows per tile
 constexpr int BLOCK_N = 128;   // kv rows per block
-constexpr int KV_SLOTS = 3;
+constexpr int KV_SLOTS = 5;
 constexpr int NUM_THREADS = 32 * (2 + 4 * NT);
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 template <int D>
 struct FwdSmem {
   static constexpr int TILE_D_BYTES = 128 * D * 2;    // Q tile, K block, V block
-  static constexpr int P_BYTES = TILE_M * BLOCK_N * 2;
-  static constexpr int Q_OFF = 0;
-  static constexpr int P_OFF = Q_OFF + NT * TILE_D_BYTES;
-  static constexpr int KV_OFF = P_OFF + NT * P_BYTES;
+  static constexpr int Q_OFF = 0;                     // a Q tile is also the staging of its output tile
+  static constexpr int KV_OFF = Q_OFF + NT * TILE_D_BYTES;
   static constexpr int BAR_OFF = KV_OFF + KV_SLOTS * TILE_D_BYTES;
   static constexpr int TOTAL = BAR_OFF + 256;
 };
@@ -56,6 +67,31 @@ struct FwdParams {
   int* status;
   b200ring::RingArgs ring;
 };
+
+// two fp32 lanes in one instruction
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 
 template <int D>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -75,7 +111,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const AbortCtx ab{abort_flag, p.status};
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   // context parallelism: the first CTAs of the grid stage K/V instead of attending
@@ -93,12 +129,31 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int hkv = h / (p.Hq / p.Hkv);
   const int q0 = qt * NT * TILE_M;
 
-  // kv block range of this CTA (kv positions are global; query row r sits at global position q_off + r)
-  int kv_begin = 0;
-  if (p.lo) kv_begin = p.lo[(long long)b * p.S + q0] / BLOCK_N;
-  int kv_end = (p.Skv + BLOCK_N - 1) / BLOCK_N;
-  if (p.causal) kv_end = min(kv_end, (p.q_off + min(q0 + NT * TILE_M, p.S) - 1) / BLOCK_N + 1);
-  const int n_blocks = is_xfer ? 0 : max(kv_end - kv_begin, 0);
+  // kv block range of each tile and of the CTA (kv positions are global; query row r sits at global position
+  // q_off + r).  The CTA streams the union; blocks are counted from its first.
+  int t_begin[NT], t_end[NT];
+  int kv_begin = 0x7fffffff, kv_end = 0;
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    const int first = q0 + t * TILE_M;
+    t_begin[t] = t_end[t] = 0;
+    if (first < p.S && !is_xfer) {
+      if (p.lo) t_begin[t] = p.lo[(long long)b * p.S + first] / BLOCK_N;
+      t_end[t] = (p.Skv + BLOCK_N - 1) / BLOCK_N;
+      if (p.causal) t_end[t] = min(t_end[t], (p.q_off + min(first + TILE_M, p.S) - 1) / BLOCK_N + 1);
+    }
+    if (t_end[t] > t_begin[t]) {
+      kv_begin = min(kv_begin, t_begin[t]);
+      kv_end = max(kv_end, t_end[t]);
+    }
+  }
+  const int n_blocks = warp_uniform(max(kv_end - kv_begin, 0));
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    if (t_end[t] <= t_begin[t]) t_begin[t] = t_end[t] = n_blocks ? kv_begin : 0;
+    t_begin[t] = warp_uniform(t_begin[t] - (n_blocks ? kv_begin : 0));
+    t_end[t] = warp_uniform(t_end[t] - (n_blocks ? kv_begin : 0));
+  }
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -169,7 +224,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n_blocks > 0) {
+    if (n_blocks > 0 && elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(TILE_M, BLOCK_N, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(TILE_M, D, false, true);
       bool ok = mbar_wait(q_full, 0, ab, ERR_WAIT_FULL);
@@ -178,11 +233,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // plus a compile-time constant in its address field (units of 16 bytes).  A tile product is D / 16 (or
       // BLOCK_N / 16) instructions of 64 clocks each and one thread issues them all, so next to nothing may sit
       // between two of them.
-      uint64_t dq[NT], dp[NT], dk[KV_SLOTS], dv[KV_SLOTS];
+      uint64_t dq[NT], dk[KV_SLOTS], dv[KV_SLOTS];
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
         dq[t] = make_smem_desc_sw128(smem_u32(smem + L::Q_OFF + t * L::TILE_D_BYTES), 16, 1024);
-        dp[t] = make_smem_desc_sw128(smem_u32(smem + L::P_OFF + t * L::P_BYTES), 16, 1024);
       }
 #pragma unroll
       for (int sl = 0; sl < KV_SLOTS; ++sl) {
@@ -190,9 +244,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         dk[sl] = make_smem_desc_sw128(kv_base, 16, 1024);
         dv[sl] = make_smem_desc_sw128(kv_base, 16384, 1024);
       }
-      static_assert(KV_SLOTS == 3 && NT == 2, "slot and tile selects below are written out");
+      auto slot_of = [](const uint64_t (&d)[KV_SLOTS], int slot) {
+        uint64_t v = d[0];
+#pragma unroll
+        for (int sl = 1; sl < KV_SLOTS; ++sl) v = slot == sl ? d[sl] : v;
+        return v;
+      };
       auto issue_qk = [&](int t, int slot) {
-        const uint64_t a0 = t == 0 ? dq[0] : dq[1], b0 = slot == 0 ? dk[0] : (slot == 1 ? dk[1] : dk[2]);
+        const uint64_t a0 = t == 0 ? dq[0] : dq[1], b0 = slot_of(dk, slot);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint64_t off = (uint64_t)(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4);
@@ -200,45 +259,53 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         tc_commit(&s_full[t]);
       };
+      // A = P in tensor memory, over the first 64 columns of S: 16 kv rows are 8 columns of packed bf16
       auto issue_pv = [&](int t, int slot, bool accumulate) {
-        const uint64_t a0 = t == 0 ? dp[0] : dp[1], b0 = slot == 0 ? dv[0] : (slot == 1 ? dv[1] : dv[2]);
+        const uint64_t b0 = slot_of(dv, slot);
 #pragma unroll
-        for (int kk = 0; kk < BLOCK_N / 16; ++kk) {
-          const uint64_t a_off = (uint64_t)(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4);
-          const uint64_t b_off = (uint64_t)((kk * 2048) >> 4);
-          tc_mma_ss(tmem_O + t * D, a0 + a_off, b0 + b_off, idesc_pv, (accumulate || kk != 0) ? 1u : 0u);
-        }
-        tc_commit(&pv_done[t]);
+        for (int kk = 0; kk < BLOCK_N / 16; ++kk)
+          tc_mma_ts(tmem_O + t * D, tmem_S + t * 128 + kk * 8, b0 + (uint64_t)((kk * 2048) >> 4), idesc_pv,
+                    (accumulate || kk != 0) ? 1u : 0u);
       };
-      if (ok) {
-        const int slot = item % KV_SLOTS;
-        ok = mbar_wait(&kv_full[slot], (item / KV_SLOTS) & 1, ab, ERR_WAIT_FULL);
-        if (ok) {
-          tc_fence_after();
-          for (int t = 0; t < NT; ++t) issue_qk(t, slot);
-          tc_commit(&kv_empty[slot]);
-          ++item;
-        }
+      auto kv_wait = [&](uint32_t it) {
+        const bool got = mbar_wait(&kv_full[it % KV_SLOTS], (it / KV_SLOTS) & 1, ab, ERR_WAIT_FULL);
+        tc_fence_after();
+        return got;
+      };
+      if (ok && (ok = kv_wait(item))) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          if (t_begin[t] == 0 && t_end[t] > 0) issue_qk(t, 0);
+        tc_commit(&kv_empty[0]);
+        ++item;
       }
       for (int j = 0; j < n_blocks && ok; ++j) {
         const bool has_next = j + 1 < n_blocks;
-        const uint32_t k_item = item;
-        const uint32_t v_item = item + (has_next ? 1 : 0);
+        const uint32_t k_item = item, v_item = item + (has_next ? 1 : 0);
         const int k_slot = k_item % KV_SLOTS, v_slot = v_item % KV_SLOTS;
-        for (int t = 0; t < NT && ok; ++t) {
-          if (!mbar_wait(&p_ready[t], j & 1, ab, ERR_WAIT_P_READY)) { ok = false; break; }
-          tc_fence_after();
-          if (has_next) {
-            if (t == 0 && !mbar_wait(&kv_full[k_slot], (k_item / KV_SLOTS) & 1, ab, ERR_WAIT_FULL)) { ok = false; break; }
-            tc_fence_after();
-            issue_qk(t, k_slot);
-            if (t == NT - 1) tc_commit(&kv_empty[k_slot]);
+        bool k_there = false, v_there = false;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          if (ok && j >= t_begin[t] && j < t_end[t]) {
+            // P(j) is in tensor memory and O is rescaled
+            ok = mbar_wait(&p_ready[t], (j - t_begin[t]) & 1, ab, ERR_WAIT_P_READY) && (v_there || kv_wait(v_item));
+            if (ok) {
+              v_there = true;
+              tc_fence_after();
+              issue_pv(t, v_slot, j > t_begin[t]);
+              if (j + 1 == t_end[t]) tc_commit(&pv_done[t]);
+            }
           }
-          if (t == 0 && !mbar_wait(&kv_full[v_slot], (v_item / KV_SLOTS) & 1, ab, ERR_WAIT_FULL)) { ok = false; break; }
-          tc_fence_after();
-          issue_pv(t, v_slot, j > 0);
-          if (t == NT - 1) tc_commit(&kv_empty[v_slot]);
+          if (ok && t == NT - 1) tc_commit(&kv_empty[v_slot]);
+          if (ok && j + 1 >= t_begin[t] && j + 1 < t_end[t]) {
+            ok = k_there || kv_wait(k_item);
+            if (ok) {
+              k_there = true;
+              issue_qk(t, k_slot);
+            }
+          }
         }
+        if (ok && has_next) tc_commit(&kv_empty[k_slot]);
         item = v_item + 1;
       }
     }
@@ -252,126 +319,122 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_sel = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t tS = tmem_S + t * 128 + lane_sel;
     const uint32_t tO = tmem_O + t * D + lane_sel;
-    uint8_t* sP = smem + L::P_OFF + t * L::P_BYTES;
+    uint8_t* sO = smem + L::Q_OFF + t * L::TILE_D_BYTES;
     int lo_row = 0;
     if (p.lo) lo_row = p.lo[(long long)b * p.S + min(q_row, p.S - 1)];
+    const int hi_row = p.causal ? min(q_pos, p.Skv - 1) : p.Skv - 1;
+    const int j_begin = t == 0 ? t_begin[0] : t_begin[1], j_end = t == 0 ? t_end[0] : t_end[1];
+    const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
     float m_ref = -1.0e30f;
     float l_sum = 0.f;
-    bool ok = n_blocks > 0;
-    for (int j = 0; j < n_blocks && ok; ++j) {
+    bool ok = j_end > j_begin;
+    for (int j = j_begin; j < j_end && ok; ++j) {
       const int kv0 = (kv_begin + j) * BLOCK_N;
-      if (!mbar_wait_warp(&s_full[t], j & 1, ab, ERR_WAIT_S_READY)) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[t], (j - j_begin) & 1, ab, ERR_WAIT_S_READY)) { ok = false; break; }
       tc_fence_after();
-      const bool need_mask = (p.causal && kv0 + BLOCK_N - 1 > q_pos) || (kv0 < lo_row) || (kv0 + BLOCK_N > p.Skv);
-      const int hi = p.causal ? min(q_pos, p.Skv - 1) : p.Skv - 1;
-      float sum = 0.f;
-      // exponentials of 32 scores relative to m_ref, their sum, and P (bf16, 128-byte swizzle, K-major for the PV
-      // MMA) into shared memory; returns the largest exponent argument seen (how far the row maximum moved)
-      auto emit_chunk = [&](const uint32_t (&r)[32], int c) -> float {
-        float e[32];
-        float top = -INFINITY;
+      const bool masked = __any_sync(0xffffffffu, kv0 + BLOCK_N - 1 > hi_row || kv0 < lo_row);
+      const int hi = hi_row - kv0, lo = lo_row - kv0;
+      auto mask = [&](uint32_t (&r)[32], int c) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float v = __uint_as_float(r[i]) * p.scale_log2 - m_ref;
-          if (need_mask) {
-            const int col = kv0 + c * 32 + i;
-            if (col > hi || col < lo_row) v = -INFINITY;
-          }
-          top = fmaxf(top, v);
-          e[i] = ex2_approx(v);
-          sum += e[i];
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint4 v;
-          v.x = pack_bf16x2(e[8 * i + 0], e[8 * i + 1]);
-          v.y = pack_bf16x2(e[8 * i + 2], e[8 * i + 3]);
-          v.z = pack_bf16x2(e[8 * i + 4], e[8 * i + 5]);
-          v.w = pack_bf16x2(e[8 * i + 6], e[8 * i + 7]);
-          const int chunk = c * 4 + i;  // 16-byte chunk index along kv (16 per row)
-          *reinterpret_cast<uint4*>(sP + (chunk >> 3) * 16384 + sw128_offset(row, chunk & 7)) = v;
-        }
-        return top;
+        for (int i = 0; i < 32; ++i)
+          if (c * 32 + i > hi || c * 32 + i < lo) r[i] = 0xff800000u;   // -inf
       };
-      // Fast path (every block but the first, unless a row maximum jumps): ONE pass over the scores with the
-      // reference maximum of the previous blocks.  The lazy-rescale rule tolerates a maximum that is up to 2^8
-      // above the reference, so the pass is kept when no row of the warp moved further; the loads of one chunk
-      // are in flight while the previous chunk is worked on.
-      bool done = false;
-      if (j > 0) {
-        if (!mbar_wait_warp(&pv_done[t], (j - 1) & 1, ab, ERR_WAIT_O_READY)) { ok = false; break; }   // P(j-1) consumed
-        // all 128 scores of the row at once: the latency of the tensor-memory loads is paid once per block
-        uint32_t ra[32], rb[32], rc[32], rd[32];
-        tmem_ld_32x32b_x32(tS, ra);
-        tmem_ld_32x32b_x32(tS + 32, rb);
-        tmem_ld_32x32b_x32(tS + 64, rc);
-        tmem_ld_32x32b_x32(tS + 96, rd);
-        tmem_ld_wait();
-        float top = emit_chunk(ra, 0);
-        top = fmaxf(top, emit_chunk(rb, 1));
-        top = fmaxf(top, emit_chunk(rc, 2));
-        top = fmaxf(top, emit_chunk(rd, 3));
-        done = !__any_sync(0xffffffffu, top > kRescaleThreshold);
-        if (!done) sum = 0.f;   // a row maximum moved too far: redo the block with a new reference
-      }
-      if (!done) {
-        // pass 1: block maximum of the scaled, masked scores
-        float bm = -INFINITY;
+      uint64_t sum0 = 0, sum1 = 0;   // two partial sums of two lanes each
+      float top;                     // largest exponent of the block relative to m_ref
+      uint32_t ra[32], rb[32], packed[64];
+      // exponentials of 32 scores relative to m_ref, their sum, and P as bf16 pairs
+      auto emit = [&](uint32_t (&r)[32], int c, uint64_t minus_m, auto is_masked) {
+        constexpr bool kMasked = decltype(is_masked)::value;
+        if constexpr (kMasked) mask(r, c);
+        float t0 = -INFINITY, t1 = -INFINITY;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(tS + c * 32, r);
-          tmem_ld_wait();
-          if (need_mask) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int col = kv0 + c * 32 + i;
-              const float v = (col > hi || col < lo_row) ? -INFINITY : __uint_as_float(r[i]);
-              bm = fmaxf(bm, v);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) bm = fmaxf(bm, __uint_as_float(r[i]));
-          }
+        for (int i = 0; i < 32; i += 4) {
+          float e0, e1, e2, e3;
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), scale2, minus_m), e0, e1);
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), scale2, minus_m), e2, e3);
+          t0 = max3(t0, e0, e1);
+          t1 = max3(t1, e2, e3);
+          e0 = ex2_approx(e0);
+          e1 = ex2_approx(e1);
+          e2 = ex2_approx(e2);
+          e3 = ex2_approx(e3);
+          sum0 = f2_add(sum0, f2_pack(e0, e1));
+          sum1 = f2_add(sum1, f2_pack(e2, e3));
+          packed[c * 16 + i / 2] = pack_bf16x2(e0, e1);
+          packed[c * 16 + i / 2 + 1] = pack_bf16x2(e2, e3);
         }
-        bm *= p.scale_log2;  // scale > 0, so the maximum commutes with it
-        const bool need = bm > m_ref + kRescaleThreshold;
-        if (__any_sync(0xffffffffu, need)) {
-          const float m_new = need ? bm : m_ref;
-          const float alpha = ex2_approx(m_ref - m_new);
-          if (j > 0) {
-            // pv_done(j-1) was waited for above: O holds the sum over the blocks before this one
-            tc_fence_after();
+        top = max3(top, t0, t1);
+      };
+      // Nearly every block but the first takes the reference maximum of the blocks before it: the lazy rule tolerates a
+      // maximum up to 2^8 above it, and whether it held is known at the end of the pass, before P goes over the scores.
+      // Otherwise the block's maximum is searched first, O and the sum are rescaled, and the pass is made again.
+      bool search = j == j_begin;
+#pragma unroll 1
+      while (true) {
+        if (search) {
+          // block maximum of the scaled scores (scale > 0, so the maximum commutes with it)
+          float bm = -INFINITY;
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            tmem_ld_32x32b_x32(tS + c * 32, ra);
+            tmem_ld_wait();
+            if (masked) mask(ra, c);
 #pragma unroll
+            for (int i = 0; i < 32; i += 2) bm = max3(bm, __uint_as_float(ra[i]), __uint_as_float(ra[i + 1]));
+          }
+          bm *= p.scale_log2;
+          const float m_new = bm > m_ref + kRescaleThreshold ? bm : m_ref;
+          const float alpha = ex2_approx(m_ref - m_new);
+          if (j > j_begin) {
+            // S(j) is complete, so PV(j-1), issued before it, is too: O holds the sum over the blocks before this one
+#pragma unroll 1
             for (int c = 0; c < D / 32; ++c) {
-              uint32_t r[32];
-              tmem_ld_32x32b_x32(tO + c * 32, r);
+              tmem_ld_32x32b_x32(tO + c * 32, ra);
               tmem_ld_wait();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-              tmem_st_32x32b_x32(tO + c * 32, r);
+              for (int i = 0; i < 32; ++i) ra[i] = __float_as_uint(__uint_as_float(ra[i]) * alpha);
+              tmem_st_32x32b_x32(tO + c * 32, ra);
             }
-            tmem_st_wait();
           }
           l_sum *= alpha;
           m_ref = m_new;
         }
-        // pass 2: probabilities, row sum, P to shared memory
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(tS + c * 32, r);
+        // one pass over the scores, the loads of 32 columns in flight while the 32 before are worked on
+        const uint64_t minus_m = f2_pack(-m_ref, -m_ref);
+        sum0 = sum1 = 0;
+        top = -INFINITY;
+        auto pass = [&](auto is_masked) {
+          tmem_ld_32x32b_x32(tS, ra);
           tmem_ld_wait();
-          emit_chunk(r, c);
-        }
+          tmem_ld_32x32b_x32(tS + 32, rb);
+          emit(ra, 0, minus_m, is_masked);
+          tmem_ld_wait();
+          tmem_ld_32x32b_x32(tS + 64, ra);
+          emit(rb, 1, minus_m, is_masked);
+          tmem_ld_wait();
+          tmem_ld_32x32b_x32(tS + 96, rb);
+          emit(ra, 2, minus_m, is_masked);
+          tmem_ld_wait();
+          emit(rb, 3, minus_m, is_masked);
+        };
+        if (masked)
+          pass(std::true_type{});
+        else
+          pass(std::false_type{});
+        if (search || !__any_sync(0xffffffffu, top > kRescaleThreshold)) break;
+        search = true;
       }
-      l_sum += sum;
-      fence_proxy_async_smem();
+      tmem_st_32x32b_x64(tS, packed);
+      float s0, s1, s2, s3;
+      f2_unpack(sum0, s0, s1);
+      f2_unpack(sum1, s2, s3);
+      l_sum += (s0 + s1) + (s2 + s3);
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[t]);
     }
-    if (ok) ok = mbar_wait_warp(&pv_done[t], (n_blocks - 1) & 1, ab, ERR_WAIT_O_READY);
+    if (ok) ok = mbar_wait_warp(&pv_done[t], 0, ab, ERR_WAIT_O_READY);
     if (ok) {
       tc_fence_after();
       const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
@@ -387,7 +450,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           v.y = pack_bf16x2(__uint_as_float(r[8 * i + 2]) * inv_l, __uint_as_float(r[8 * i + 3]) * inv_l);
           v.z = pack_bf16x2(__uint_as_float(r[8 * i + 4]) * inv_l, __uint_as_float(r[8 * i + 5]) * inv_l);
           v.w = pack_bf16x2(__uint_as_float(r[8 * i + 6]) * inv_l, __uint_as_float(r[8 * i + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(sP + (c >> 1) * 16384 + sw128_offset(row, (c & 1) * 4 + i)) = v;
+          *reinterpret_cast<uint4*>(sO + (c >> 1) * 16384 + sw128_offset(row, (c & 1) * 4 + i)) = v;
         }
       }
       fence_proxy_async_smem();
@@ -395,7 +458,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int slab_row = q0 + t * TILE_M + quad * 32;
       if (lane == 0 && slab_row < p.S) {
         for (int bx = 0; bx < NBOX; ++bx)
-          tma_store_4d(&tmO, sP + bx * 16384 + quad * 32 * 128, bx * 64, h, slab_row, b);
+          tma_store_4d(&tmO, sO + bx * 16384 + quad * 32 * 128, bx * 64, h, slab_row, b);
         tma_commit_group();
         tma_wait_group<0>();
       }

@@ -62,6 +62,69 @@ def test_attn_fwd(D, S, causal, docs):
     assert torch.allclose(o.float(), ref_o, atol=2e-2, rtol=2e-2), (o.float() - ref_o).abs().max()
 
 
+def _exact(q, k, v, causal, lo):
+    """64-bit attention, one head at a time."""
+
+    B, S, Hq, D = q.shape
+    g = Hq // k.shape[2]
+    at = torch.arange(S, device=q.device)
+    hidden = (at[None, :] > at[:, None]).expand(B, S, S) if causal else torch.zeros(B, S, S, dtype=torch.bool, device=q.device)
+    if lo is not None:
+        hidden = hidden | (at[None, None, :] < lo[:, :, None])
+    o = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    lse = torch.empty((B, Hq, S), dtype=torch.float64, device=q.device)
+    for b in range(B):
+        for h in range(Hq):
+            s = (q[b, :, h].double() @ k[b, :, h // g].double().T * D ** -0.5).masked_fill(hidden[b], float("-inf"))
+            lse[b, h] = torch.logsumexp(s, -1)
+            o[b, :, h] = s.softmax(-1) @ v[b, :, h // g].double()
+    return o, lse
+
+
+# lengths around the edges of a 128-row tile, a CTA's two tiles and the ring of kv blocks; documents that start inside
+# and between tiles, so that the two tiles of a CTA see different blocks
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("S", [1, 127, 128, 129, 255, 257, 385, 900, 1408])
+@pytest.mark.parametrize("kind", ["causal", "full", "docs", "window", "cuts"])
+def test_attn_fwd_edges(D, S, kind):
+    from research_b200.ops import native
+
+    B, Hq, Hkv = 2, 3, 1
+    q, k, v = _bf((B, S, Hq, D), 11), _bf((B, S, Hkv, D), 12), _bf((B, S, Hkv, D), 13)
+    at = torch.arange(S, device="cuda", dtype=torch.int32)
+    lo = {"causal": None, "full": None, "docs": doc_lo(B, S, 90, 5), "window": (at - 99).clamp_min(0).expand(B, S),
+          "cuts": (at // 128 * 128).expand(B, S)}[kind]
+    lo = None if lo is None else lo.contiguous()
+    o, lse = native.attn_fwd(q, k, v, causal=kind != "full", lo=lo)
+    ref_o, ref_lse = _exact(q, k, v, kind != "full", lo)
+    native.check_status()
+    # P and o are rounded to bf16 (2^-9 each); scores are fp32 sums of 128 products
+    assert (o.double() - ref_o).norm() / ref_o.norm() < 2.0 ** -8
+    assert (lse.double() - ref_lse).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("D", [128, 64])
+def test_attn_fwd_jumping_maxima_and_nonfinite(D):
+    """Row maxima that jump by far more than the lazy rule tolerates, late and more than once; a NaN in one key reaches
+    the rows that see it and no others."""
+
+    from research_b200.ops import native
+
+    B, S, H = 1, 1024, 2
+    q, k, v = _bf((B, S, H, D), 21), _bf((B, S, H, D), 22), _bf((B, S, H, D), 23)
+    for at, mul in ((130, 4.0), (400, 9.0), (401, 16.0), (900, 30.0)):
+        k[:, at] = (k[:, at].float() * mul).to(torch.bfloat16)
+    o, lse = native.attn_fwd(q, k, v)
+    ref_o, ref_lse = _exact(q, k, v, True, None)
+    assert (o.double() - ref_o).norm() / ref_o.norm() < 2.0 ** -8
+    assert ((lse.double() - ref_lse).abs() / ref_lse.abs().clamp_min(1)).max() < 1e-4
+    k[:, 700, 1] = float("nan")
+    o, _ = native.attn_fwd(q, k, v)
+    native.check_status()
+    assert torch.isfinite(o[:, :, 0]).all() and torch.isfinite(o[:, :700, 1]).all()
+    assert torch.isnan(o[:, 700:, 1]).all()
+
+
 def test_attn_fwd_sliding_window_and_speed():
     from research_b200.ops import native
 
