@@ -110,7 +110,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const AbortCtx ab{abort_flag, p.status};
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const int G = p.Hq / p.Hkv;
   const int q_tiles = (p.S + TILE - 1) / TILE;
@@ -156,6 +156,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
       n_total = blk_count * G;
     }
     if (is_xfer) blk_count = n_total = 0;
+    n_total = warp_uniform(n_total);   // selects the ring slots of the MMA descriptors
   }
   const int hkv = DKV ? h_res : h_res / G;
 
@@ -236,7 +237,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n_total > 0) {
+    if (n_total > 0 && elect_one()) {
       constexpr uint32_t idesc_t = make_idesc_bf16(TILE, TILE, false, false);  // X * Y^T, both K-major over D
       constexpr uint32_t idesc_a = make_idesc_bf16(TILE, D, false, true);      // K-major A * Y (MN-major)
       auto ybuf = [&](int item) -> const uint8_t* { return smem + L::RING_OFF + (item % RING) * L::TILE_BYTES; };

@@ -87,7 +87,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile unsigned int* fin_prev = reinterpret_cast<volatile unsigned int*>(tmem_slot + 2);
   const AbortCtx ab{abort_flag, p.status};
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   const int tiles_m = (p.M + BM - 1) / BM;
@@ -213,9 +213,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
-      uint32_t it = 0;
+      uint32_t s = 0, ph = 0;
       uint32_t tile_iter = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
@@ -228,22 +228,20 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!mbar_wait(&tempty[acc], acc_ph ^ 1, ab, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full[s], ph, ab, ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_base = smem_u32(smem + s * L::STAGE_BYTES);
-          const uint32_t b_base = a_base + A_TILE_BYTES;
+          const uint64_t adesc = make_smem_desc_sw128(a_base, A_MN ? 8192 : 16, 1024);
+          const uint64_t bdesc = make_smem_desc_sw128(a_base + A_TILE_BYTES, B_MN ? 8192 : 16, 1024);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = make_smem_desc_sw128(a_base + (A_MN ? k * 2048 : k * 32), A_MN ? 8192 : 16, 1024);
-            const uint64_t bdesc = make_smem_desc_sw128(b_base + (B_MN ? k * 2048 : k * 32), B_MN ? 8192 : 16, 1024);
-            tc_mma_ss(d_tmem, adesc, bdesc, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
-          }
-          tc_commit(&empty[s]);  // stage reusable once these MMAs have read it
+          for (int k = 0; k < BK / 16; ++k)
+            tc_mma_ss(d_tmem, adesc + (A_MN ? k * 128 : k * 2), bdesc + (B_MN ? k * 128 : k * 2), idesc,
+                      (kb != kb0 || k != 0) ? 1u : 0u);
+          tc_commit(&empty[s]);
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
-        if (ok) tc_commit(&tfull[acc]);  // accumulator complete
+        if (ok) tc_commit(&tfull[acc]);
       }
     }
   } else {
@@ -399,7 +397,8 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
                      int batch_c, long long lda, long long ldb, long long ldc, long long stride_a, long long stride_b,
                      long long stride_c, int a_mn, int b_mn, int out_f32, int accumulate, int bn_hint,
                      const int* tile_group, const int* k_range, int* status, void* stream, int c_shared = 0,
-                     void* fin_out = nullptr, long long fin_ld_out = 0, void* fin_count = nullptr, int pdl = 0);
+                     void* fin_out = nullptr, long long fin_ld_out = 0, void* fin_count = nullptr, int pdl = 0,
+                     int k_total = 0);
 
 extern "C" int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int batch, long long lda,
                               long long ldb, long long ldc, long long stride_a, long long stride_b,
@@ -433,14 +432,17 @@ extern "C" int b200_gemm_bf16_splitk_fused(const void* A, const void* B, void* w
 }
 
 // Split-K for any operand layout with an fp32 output that is accumulated into (weight gradients: the contraction
-// runs over tokens and is long, the output has few tiles, and the partial sums are reduce-added anyway).
+// runs over tokens and is long, the output has few tiles, and the partial sums are reduce-added anyway).  Slices are
+// whole 64-element blocks of K; the last may be shorter.
 extern "C" int b200_gemm_bf16_splitk_acc(const void* A, const void* B, void* C, int M, int N, int K, int splits,
                                          long long lda, long long ldb, long long ldc, int a_mn, int b_mn, int* status,
                                          void* stream) {
-  if (splits < 1 || K % (64 * splits)) return b200host::RC_BAD_SHAPE;
-  const int kc = K / splits;
-  return gemm_impl(A, B, C, M, N, kc, splits, 1, 1, 1, lda, ldb, ldc, 0, 0, 0, a_mn, b_mn, 1, 1, 0, nullptr, nullptr,
-                   status, stream, 1);
+  if (splits < 1 || K < 1) return b200host::RC_BAD_SHAPE;
+  const int blocks = (K + BK - 1) / BK;
+  const int per = (blocks + splits - 1) / splits;
+  splits = (blocks + per - 1) / per;   // no slice is empty
+  return gemm_impl(A, B, C, M, N, per * BK, splits, 1, 1, 1, lda, ldb, ldc, 0, 0, 0, a_mn, b_mn, 1, 1, 0, nullptr,
+                   nullptr, status, stream, 1, nullptr, 0, nullptr, 0, K);
 }
 
 // Grouped forward / data-gradient product: A [M_pad, K] and C [M_pad, N] are 2-D with every group's rows
@@ -466,14 +468,15 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
                      int batch_c, long long lda, long long ldb, long long ldc, long long stride_a, long long stride_b,
                      long long stride_c, int a_mn, int b_mn, int out_f32, int accumulate, int bn_hint,
                      const int* tile_group, const int* k_range, int* status, void* stream, int c_shared, void* fin_out,
-                     long long fin_ld_out, void* fin_count, int pdl) {
+                     long long fin_ld_out, void* fin_count, int pdl, int k_total) {
   using namespace b200host;
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return RC_BAD_SHAPE;
   const int BN = (bn_hint == 128 || bn_hint == 256) ? bn_hint : (N > 128 ? 256 : 128);
   CUtensorMap tmA, tmB, tmC;
   int rc;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  const int k_map = c_shared ? K * batch : K;  // split-K addresses slices through the K coordinate
+  // split-K addresses slices through the K coordinate; what lies past the end of K reads as zero
+  const int k_map = k_total ? k_total : (c_shared ? K * batch : K);
   if (c_shared) batch_a = batch_b = batch_c = 1;
   if (!a_mn)
     rc = make_map_3d(&tmA, bf, A, k_map, M, batch_a, lda * 2, stride_a * 2, BK, BM);
