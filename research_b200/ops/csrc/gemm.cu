@@ -17,6 +17,12 @@
 // transpose pass.  No cluster launch and no multicast loads: the same code runs on any number of
 // GPUs.  The role this plays in the reference is XLA's cuBLAS dot; the hand-written comparator in
 // its vendored tree is third_party/ThunderKittens/kernels/gemm/bf16_b200/bf16_b200_gemm.cu.
+//
+// SYM: the output is a product of a matrix with its own transpose (the Gram and the square of a Gram of a Newton-Schulz
+// step): only output tiles that reach the diagonal or lie right of it are computed, and the epilogue writes a tile's
+// transpose as well, half the tiles for the same result bit for bit.  It can add a multiple of the (symmetric) input and
+// of the identity on the way out, which makes a Newton-Schulz step three launches without an element-wise pass.
+// Eight matrices of 2048 x 2048: a Gram 106 -> 71 us, five steps 1823 -> 1248 us; of 5632 x 2048: 3566 -> 2644 us.
 #include "b200.cuh"
 #include "host_util.cuh"
 
@@ -66,9 +72,23 @@ struct GemmParams {
   // Programmatic dependent launch (skinny split-K products of a decode step): the weight tiles of the first stages
   // are requested before the wait for the predecessor, only the activation tiles and the output come after it.
   int pdl;
+  // SYM: C = alpha * acc + beta * G + gamma * I, written with its transpose; G (nullptr: none) and C share their strides.
+  const __nv_bfloat16* sym_g;
+  __nv_bfloat16* sym_c;
+  long long sym_ld, sym_stride;
+  float sym_alpha, sym_beta, sym_gamma;
 };
 
-template <int BN, bool A_MN, bool B_MN, bool OUT_F32>
+// Output tiles of one SYM matrix, column by column: column j (BN wide) has the row tiles 0 .. R (j + 1) - 1, R = BN / BM.
+template <int BN>
+__host__ __device__ constexpr int sym_tiles_before(int j) { return (BN / BM) * j * (j + 1) / 2; }
+template <int BN>
+__host__ __device__ constexpr int sym_tiles(int tiles_m, int tiles_n) {
+  const int last = (BN / BM) * tiles_n;
+  return sym_tiles_before<BN>(tiles_n - 1) + (last < tiles_m ? last : tiles_m);
+}
+
+template <int BN, bool A_MN, bool B_MN, bool OUT_F32, bool SYM = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
@@ -92,7 +112,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   const int tiles_m = (p.M + BM - 1) / BM;
   const int tiles_n = (p.N + BN - 1) / BN;
-  const int per_batch = tiles_m * tiles_n;
+  const int per_batch = SYM ? sym_tiles<BN>(tiles_m, tiles_n) : tiles_m * tiles_n;
   const int total_tiles = per_batch * p.batch;
   const int k_blocks = (p.K + BK - 1) / BK;
 
@@ -138,6 +158,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   auto tile_coords = [&](int t, int& b, int& m0, int& n0) {
     b = t / per_batch;
     const int r = t - b * per_batch;
+    if constexpr (SYM) {
+      int j = (int)((sqrtf((float)(8 / (BN / BM) * r + 1)) - 1.f) * 0.5f);
+      while (sym_tiles_before<BN>(j + 1) <= r) ++j;
+      while (sym_tiles_before<BN>(j) > r) --j;
+      m0 = (r - sym_tiles_before<BN>(j)) * BM;
+      n0 = j * BN;
+      return;
+    }
     const int group_size = GROUP_M * tiles_n;
     const int g = r / group_size;
     const int first_m = g * GROUP_M;
@@ -284,6 +312,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           for (int h = 0; h < 2; ++h) {
             uint32_t r[32];
             tmem_ld_32x32b_x32(t_row + j * 64 + h * 32, r);
+            if constexpr (SYM) {
+              const int row = row0 + lane;
+              uint4 g[4];
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const int col = col0 + h * 32 + c * 8;
+                g[c] = make_uint4(0, 0, 0, 0);
+                if (p.sym_g && row < p.M && col < p.N)
+                  g[c] = *reinterpret_cast<const uint4*>(p.sym_g + b * p.sym_stride + row * p.sym_ld + col);
+              }
+              tmem_ld_wait();
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&g[c]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  const float gv = (i & 1) ? __high2float(gh[i >> 1]) : __low2float(gh[i >> 1]);
+                  float v = fmaf(p.sym_beta, gv, p.sym_alpha * __uint_as_float(r[8 * c + i]));
+                  if (col0 + h * 32 + c * 8 + i == row) v += p.sym_gamma;
+                  r[8 * c + i] = __float_as_uint(v);
+                }
+              }
+            }
             tmem_ld_wait();
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -305,6 +356,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           else
             tma_store_3d(&tmC, buf, col0, row0, zC);
           tma_commit_group();
+        }
+        if constexpr (SYM) {
+          // the transposed 64 x 32 piece, unless it lies in a tile that is computed: right of the diagonal block, and
+          // not the second block of the diagonal tile (its rows are that tile's last 128)
+          const int mb = m0 / BM, cb = col0 / BM;
+          if (cb > mb && !(BN == 256 && (mb & 1) == 0 && cb == mb + 1)) {
+            const int part = lane & 3, grow = row0 + part * 8;
+#pragma unroll 2
+            for (int c8 = 0; c8 < 8; ++c8) {
+              const int c = c8 * 8 + (lane >> 2), gcol = col0 + c;
+              uint32_t w[4];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint32_t v = *reinterpret_cast<const uint16_t*>(buf + sw128_offset(part * 8 + i, c >> 3) + (c & 7) * 2);
+                w[i >> 1] = (i & 1) ? (w[i >> 1] | (v << 16)) : v;
+              }
+              if (gcol < p.N && grow < p.M)
+                *reinterpret_cast<uint4*>(p.sym_c + b * p.sym_stride + gcol * p.sym_ld + grow) =
+                    make_uint4(w[0], w[1], w[2], w[3]);
+            }
+          }
         }
       }
       // every tcgen05.ld of this accumulator has completed: hand it back to the MMA issuer
@@ -357,11 +429,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
-template <int BN, bool A_MN, bool B_MN, bool OUT_F32>
+template <int BN, bool A_MN, bool B_MN, bool OUT_F32, bool SYM = false>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const GemmParams& p, int grid,
            cudaStream_t stream) {
   using L = SmemLayout<BN>;
-  auto* kern = gemm_bf16_kernel<BN, A_MN, B_MN, OUT_F32>;
+  auto* kern = gemm_bf16_kernel<BN, A_MN, B_MN, OUT_F32, SYM>;
   constexpr int smem_bytes = L::TOTAL + 1024;
   static bool configured[b200host::kMaxDevices] = {};   // per kernel instantiation and device
   if (int rc = b200host::ensure_dynamic_smem(kern, smem_bytes, configured)) return rc;
@@ -443,6 +515,47 @@ extern "C" int b200_gemm_bf16_splitk_acc(const void* A, const void* B, void* C, 
   splits = (blocks + per - 1) / per;   // no slice is empty
   return gemm_impl(A, B, C, M, N, per * BK, splits, 1, 1, 1, lda, ldb, ldc, 0, 0, 0, a_mn, b_mn, 1, 1, 0, nullptr,
                    nullptr, status, stream, 1, nullptr, 0, nullptr, 0, K);
+}
+
+// C[b] = alpha * A[b] A[b]^T + beta * G[b] + gamma * I for a stack of matrices, each C[b] a symmetric d x d matrix of
+// which only the tiles on and right of the diagonal are computed.  a_mn = 0: A is [batch, d, K]; a_mn = 1: A is
+// [batch, K, d] (the product is A^T A).  G (optional) is laid out as C; strides in elements, multiples of 8.
+extern "C" int b200_gemm_bf16_sym(const void* A, const void* G, void* C, int d, int K, int batch, long long lda,
+                                  long long ldc, long long stride_a, long long stride_c, int a_mn, float alpha,
+                                  float beta, float gamma, int* status, void* stream) {
+  using namespace b200host;
+  if (d <= 0 || K <= 0 || batch <= 0 || d % 8 || (stride_c & 7) || (ldc & 7)) return RC_BAD_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(G) & 15)) return RC_BAD_ALIGNMENT;
+  const int rows = (d + BM - 1) / BM;
+  const int t128 = sym_tiles<128>(rows, rows) * batch, t256 = sym_tiles<256>(rows, (d + 255) / 256) * batch;
+  // a 128-wide tile takes a little more than half the time of a 256-wide one: whichever leaves the shorter last wave
+  const int sms = sm_count();
+  const bool narrow = d <= 128 || 0.55f * ((t128 + sms - 1) / sms) < (float)((t256 + sms - 1) / sms);
+  const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  CUtensorMap tmA, tmB, tmC;
+  int rc;
+  if (!a_mn) {
+    if ((rc = make_map_3d(&tmA, bf, A, K, d, batch, lda * 2, stride_a * 2, BK, BM))) return rc;
+    if ((rc = make_map_3d(&tmB, bf, A, K, d, batch, lda * 2, stride_a * 2, BK, narrow ? 128 : 256))) return rc;
+  } else {
+    if ((rc = make_map_3d(&tmA, bf, A, d, K, batch, lda * 2, stride_a * 2, 64, BK))) return rc;
+    tmB = tmA;
+  }
+  if ((rc = make_map_3d(&tmC, bf, C, d, d, batch, ldc * 2, stride_c * 2, 64, 32))) return rc;
+  GemmParams p{d, d, K, batch, 0, status};
+  p.sym_g = static_cast<const __nv_bfloat16*>(G);
+  p.sym_c = static_cast<__nv_bfloat16*>(C);
+  p.sym_ld = ldc;
+  p.sym_stride = stride_c;
+  p.sym_alpha = alpha;
+  p.sym_beta = beta;
+  p.sym_gamma = gamma;
+  const int tiles = narrow ? t128 : t256, grid = tiles < sms ? tiles : sms;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (narrow) return a_mn ? launch<128, true, true, false, true>(tmA, tmB, tmC, p, grid, s)
+                          : launch<128, false, false, false, true>(tmA, tmB, tmC, p, grid, s);
+  return a_mn ? launch<256, true, true, false, true>(tmA, tmB, tmC, p, grid, s)
+              : launch<256, false, false, false, true>(tmA, tmB, tmC, p, grid, s);
 }
 
 // Grouped forward / data-gradient product: A [M_pad, K] and C [M_pad, N] are 2-D with every group's rows

@@ -80,6 +80,8 @@ def _declare(lib: ctypes.CDLL) -> None:
 
     sig("b200_gemm_bf16", c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_ll, c_ll, c_ll,
         c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p)
+    sig("b200_gemm_bf16_sym", c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_ll, c_int, c_float,
+        c_float, c_float, c_void_p, c_void_p)
     sig("b200_rmsnorm_fwd", c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p)
     sig("b200_rmsnorm_bwd", c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p)
     sig("b200_qknorm_rope_fwd", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_int, c_void_p, c_void_p, c_ll, c_int, c_int,
@@ -262,6 +264,27 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         int(trans_a), int(not trans_b), int(out.dtype == torch.float32), int(accumulate), bn,
         status_word(a.device).data_ptr(), _stream())
     _check(rc, "b200_gemm_bf16")
+    return out
+
+
+def gram(x: torch.Tensor, *, transposed: bool = False, alpha: float = 1.0, beta: float = 0.0,
+         gamma: float = 0.0) -> torch.Tensor:
+    """``alpha * x x^T + beta * x + gamma * I`` (``transposed``: of ``x^T x``) for a contiguous bf16 stack ``[batch, m, n]``
+    with m and n multiples of 8; the result is symmetric bit for bit and half of it is computed.  ``beta`` needs a
+    stack of symmetric matrices."""
+
+    lib = load()
+    if x.dtype != torch.bfloat16 or x.dim() != 3 or not x.is_contiguous() or x.shape[1] % 8 or x.shape[2] % 8:
+        raise KernelError(f"gram needs a contiguous bf16 [batch, m, n] stack with m, n % 8 == 0, got {tuple(x.shape)}")
+    batch, m, n = x.shape
+    d, K = (n, m) if transposed else (m, n)
+    if beta != 0.0 and m != n:
+        raise KernelError("gram: beta adds the input itself, which has to be square")
+    out = torch.empty((batch, d, d), dtype=x.dtype, device=x.device)
+    rc = lib.b200_gemm_bf16_sym(x.data_ptr(), x.data_ptr() if beta != 0.0 else None, out.data_ptr(), d, K, batch, n, d,
+                                m * n, d * d, int(transposed), alpha, beta, gamma,
+                                status_word(x.device).data_ptr(), _stream())
+    _check(rc, "b200_gemm_bf16_sym")
     return out
 
 

@@ -70,22 +70,15 @@ def _iterate(x: torch.Tensor, coefficients) -> torch.Tensor:
 
 
 def newton_schulz_stack_(x: torch.Tensor, coefficients=None) -> torch.Tensor:
-    """Newton-Schulz on an already normalised bf16 stack ``[batch, m, n]`` with three batched tcgen05 GEMMs per step.
-
-    Uses ``a X + (b G + c G^2) X = ((b I + c G) G + a I) X`` so that no step needs an accumulate pass:
-    ``G = X X^T`` (or ``X^T X`` when tall), ``Q = (b I + c G) G``, ``X <- (Q + a I) X``.
-    """
+    """Newton-Schulz on an already normalised bf16 stack ``[batch, m, n]`` with three batched tcgen05 GEMMs per step:
+    ``G = X X^T`` (or ``X^T X`` when tall), ``Q = c G G^T + b G + a I``, ``X <- Q X``.  G and Q are symmetric: half of
+    their tiles are computed and the polynomial is formed as Q leaves the product."""
 
     coefficients = coefficients or (MUON_NS_COEFFICIENTS,) * MUON_NS_STEPS
     tall = x.shape[-2] > x.shape[-1]
     for a, b, c in coefficients:
-        if tall:
-            gram = native.gemm(x, x, trans_a=True, trans_b=False)
-        else:
-            gram = native.gemm(x, x, trans_b=True)
-        lhs = native.affine_identity(gram, b, c)                  # b I + c G
-        q = native.gemm(lhs, gram, trans_b=True)                  # G symmetric: (bI + cG) G^T = bG + cG^2
-        native.affine_identity(q, a, 1.0, out=q)                  # + a I
+        g = native.gram(x, transposed=tall)
+        q = native.gram(g, alpha=c, beta=b, gamma=a)
         if tall:
             x = native.gemm(x, q, trans_b=True)                   # X Q   (Q symmetric)
         else:

@@ -98,8 +98,8 @@ def test_attn_fwd_edges(D, S, kind):
     o, lse = native.attn_fwd(q, k, v, causal=kind != "full", lo=lo)
     ref_o, ref_lse = _exact(q, k, v, kind != "full", lo)
     native.check_status()
-    # P and o are rounded to bf16 (2^-9 each); scores are fp32 sums of 128 products
-    assert (o.double() - ref_o).norm() / ref_o.norm() < 2.0 ** -8
+    # P and o are rounded to bf16 (2^-8 of a value at most, each); scores are fp32 sums of 128 products
+    assert (o.double() - ref_o).norm() / ref_o.norm() < 2.0 ** -7
     assert (lse.double() - ref_lse).abs().max() < 1e-4
 
 
@@ -116,7 +116,7 @@ def test_attn_fwd_jumping_maxima_and_nonfinite(D):
         k[:, at] = (k[:, at].float() * mul).to(torch.bfloat16)
     o, lse = native.attn_fwd(q, k, v)
     ref_o, ref_lse = _exact(q, k, v, True, None)
-    assert (o.double() - ref_o).norm() / ref_o.norm() < 2.0 ** -8
+    assert (o.double() - ref_o).norm() / ref_o.norm() < 2.0 ** -7
     assert ((lse.double() - ref_lse).abs() / ref_lse.abs().clamp_min(1)).max() < 1e-4
     k[:, 700, 1] = float("nan")
     o, _ = native.attn_fwd(q, k, v)

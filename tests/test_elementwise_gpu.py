@@ -82,8 +82,8 @@ def test_rmsnorm_bwd_widths(H, rows, with_res):
     (xr * torch.rsqrt(xr.pow(2).mean(-1, keepdim=True) + 1e-6) * wr).backward(dy.double())
     dw = torch.ones(H, device="cuda")                                   # accumulated into
     dx = native.rmsnorm_bwd(x, w, rstd, dy, dw, dres)
-    # one rounding to bf16 (2^-9 of each value); fp32 sums of at most 1203 terms (2^-24 each) on top of the 1
-    assert _off(dx, xr.grad + (0 if dres is None else dres.double())) < 2.0 ** -9
+    # one rounding to bf16 (2^-8 of each value at most); fp32 sums of at most 1203 terms (2^-24 each) on top of the 1
+    assert _off(dx, xr.grad + (0 if dres is None else dres.double())) < 2.0 ** -8
     assert _off(dw, wr.grad + 1) < 1e-5
 
 
@@ -110,8 +110,8 @@ def test_qknorm_rope_shapes(T, hq, hkv, D):
     native.qknorm_rope_bwd_qk(buf, same, same, wq, wk, pos, r, torch.zeros_like(dq), torch.zeros_like(dk), hq, hkv, D,
                               10000.0, True)
     # one rounding to bf16; the angle is formed in fp32: 251 * 2^-24 = 1.5e-5
-    assert _off(out.view(T, hq + hkv, D), ref) < 2.0 ** -9
-    assert _off(din[:, :(hq + hkv) * D].view(T, hq + hkv, D), grads[0]) < 2.0 ** -9
+    assert _off(out.view(T, hq + hkv, D), ref) < 2.0 ** -8
+    assert _off(din[:, :(hq + hkv) * D].view(T, hq + hkv, D), grads[0]) < 2.0 ** -8
     assert _off(dq, grads[1]) < 1e-4 and _off(dk, grads[2]) < 1e-4
     assert torch.equal(same, din[:, :(hq + hkv) * D]) and not din[:, (hq + hkv) * D:].any()
 

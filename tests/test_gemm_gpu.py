@@ -134,3 +134,29 @@ def test_weight_gradient_with_ragged_tokens(tokens, m, n):
     ref = 0.25 + dy.double().t() @ x.double()
     # exact products, fp32 sums of at most 2999 of them in any order: 2999 * 2^-24 of the sum of magnitudes, far from reached
     assert (grad.double() - ref).abs().max() <= 2.0 ** -18 * (dy.double().abs().t() @ x.double().abs()).max() + 2.0 ** -24
+
+
+# sizes around the edges of a 128-row block and of the narrow and the wide tile, odd numbers of blocks, both operand
+# layouts; batches that make the launcher take either tile width
+@pytest.mark.parametrize("d", [8, 64, 128, 136, 256, 384, 520, 1024, 1160])
+@pytest.mark.parametrize("K", [8, 200, 512])
+@pytest.mark.parametrize("batch", [1, 3, 20])
+def test_gram_is_symmetric_and_exact(d, K, batch):
+    from research_b200.ops import native
+
+    torch.manual_seed(d + K)
+    for transposed in (False, True):
+        x = (torch.randn((batch, K, d) if transposed else (batch, d, K), device="cuda") * 0.1).bfloat16()
+        g = native.gram(x, transposed=transposed)
+        xd = x.double().transpose(1, 2) if transposed else x.double()
+        ref = xd @ xd.transpose(1, 2)
+        assert torch.equal(g, g.transpose(1, 2))
+        assert (g.double() - ref).norm() <= 2.0 ** -8 * ref.norm()       # one rounding to bf16: 2^-8 of a value at most
+    q = native.gram(g, alpha=2.0, beta=-4.75, gamma=3.5)
+    gd = g.double()
+    ref = 2.0 * gd @ gd - 4.75 * gd + 3.5 * torch.eye(d, device="cuda", dtype=torch.float64)
+    native.check_status()
+    assert torch.equal(q, q.transpose(1, 2))
+    assert (q.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+    with pytest.raises(native.KernelError):
+        native.gram(x[:, :, :4] if d != 4 else x)
