@@ -10,6 +10,7 @@ components/attention.py:213-218).
 
 from __future__ import annotations
 
+from contextlib import contextmanager
 from dataclasses import dataclass
 
 import torch
@@ -33,6 +34,18 @@ class PagedKVCache:
         self.page_table = torch.arange(total_pages, device=device, dtype=torch.int32).view(batch, self.pages_per_seq)
         self.lengths = torch.zeros(batch, dtype=torch.int32, device=device)
         self.batch = batch
+        self._from_zero = False
+
+    @contextmanager
+    def prompt(self):
+        """For a caller that writes rows ``0, 1, 2, ...`` of every sequence (a prompt into an empty cache): inside, the
+        layers take that as given instead of reading the positions back from the device, which would wait for it."""
+
+        before, self._from_zero = self._from_zero, True
+        try:
+            yield self
+        finally:
+            self._from_zero = before
 
     def _pages(self, pool: torch.Tensor, layer: int) -> torch.Tensor:
         # with the identity page table, sequence b owns pages [b * pages_per_seq, (b + 1) * pages_per_seq)
@@ -65,7 +78,21 @@ class PagedKVCache:
             lo = None if window is None else (pos - (window - 1)).clamp_min(0).to(torch.int32)
             return decode_attention_paged(q[:, 0], kp, vp, lengths, lo)[:, None]
         idx = positions.long()
-        from_zero = T > 1 and bool((positions == torch.arange(T, device=q.device, dtype=positions.dtype)).all())
+        from_zero = T > 1 and (self._from_zero or bool(
+            (positions == torch.arange(T, device=q.device, dtype=positions.dtype)).all()))
+        if from_zero and native_ok and kp.dtype == torch.bfloat16:
+            # prefill from position 0: the rows go to their pages in one launch and the flash kernel takes them where
+            # they are (column ranges of the packed projection)
+            from research_b200.ops import native
+            from research_b200.ops.decode import kv_write_prompt_paged
+
+            q, k, v = (t if _packed_view(t) else t.contiguous() for t in (q, k, v))
+            kv_write_prompt_paged(k, v, kp, vp)
+            lo = None
+            if window is not None:
+                lo = (positions - (window - 1)).clamp_min(0).to(torch.int32).contiguous()
+            o, _ = native.attn_fwd(q, k, v, causal=True, lo=lo)
+            return o.reshape(B, T, -1)
         if from_zero:
             # a prompt written from row 0: whole pages are strided block copies, no index arithmetic per element
             ps = self.page_size
@@ -82,7 +109,6 @@ class PagedKVCache:
             kp[b_idx, idx // self.page_size, :, idx % self.page_size] = k.to(kp.dtype)
             vp[b_idx, idx // self.page_size, :, idx % self.page_size] = v.to(vp.dtype)
         if from_zero and native_ok:
-            # prefill from position 0: the flash kernel over the rows just computed
             from research_b200.ops import native
 
             lo = None
@@ -100,6 +126,13 @@ class PagedKVCache:
 
     def advance(self, positions: torch.Tensor) -> None:
         self.lengths = torch.maximum(self.lengths, (positions.max(dim=1).values + 1).to(torch.int32))
+
+
+def _packed_view(t: torch.Tensor) -> bool:
+    """Whether the flash and cache kernels can read ``[B, T, heads, D]`` in place: dense heads, 16-byte rows."""
+
+    return (t.dtype == torch.bfloat16 and t.stride(3) == 1 and t.stride(2) == t.shape[3] and t.stride(1) % 8 == 0
+            and t.stride(1) >= t.shape[2] * t.shape[3] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
 
 
 def _masked_attention(q, k, v, allowed):
@@ -198,7 +231,8 @@ def prefill(model, prompt_ids: torch.Tensor, cache: PagedKVCache) -> torch.Tenso
     B, P = prompt_ids.shape
     device = next(model.parameters()).device
     positions = torch.arange(P, device=device, dtype=torch.int32).expand(B, P).contiguous()
-    logits = model.run_with_cache(prompt_ids.to(device=device, dtype=torch.int32), positions, cache, last_only=True)
+    with cache.prompt():
+        logits = model.run_with_cache(prompt_ids.to(device=device, dtype=torch.int32), positions, cache, last_only=True)
     cache.advance(positions)
     return logits[:, -1]
 
@@ -242,7 +276,8 @@ def generate_tokens(model, prompt_ids: torch.Tensor, *, max_new_tokens: int, tem
     cache = init_kv_cache(model, B, total, page_size=page_size)
     gen = torch.Generator(device=device).manual_seed(int(seed))
     positions = torch.arange(P, device=device, dtype=torch.int32).expand(B, P).contiguous()
-    logits = model.run_with_cache(prompt_ids.to(torch.int32), positions, cache, last_only=True)[:, -1]
+    with cache.prompt():
+        logits = model.run_with_cache(prompt_ids.to(torch.int32), positions, cache, last_only=True)[:, -1]
     cache.advance(positions)
     tokens, logprobs = [], []
     step = None

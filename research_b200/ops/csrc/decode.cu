@@ -219,6 +219,27 @@ __global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ k_new, const 
   }
 }
 
+// A prompt into empty caches: rows 0 .. T-1 of every sequence, K and V in one launch, read where the projection left
+// them.  One thread per 8 elements, so a warp moves two heads' rows of 128 elements; bound by launch latency at the
+// sizes of a single prompt (four strided copies and three dense ones per layer took 25 us of 777 rows, this 4 us).
+__global__ void kv_write_prompt_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
+                                       long long k_row, long long k_batch, long long v_row, long long v_batch,
+                                       __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
+                                       long long c_batch, long long c_head, long long c_page, int page_rows, int B,
+                                       int T, int Hkv, int D) {
+  const int per = D / 8, per_row = per * Hkv;
+  const long long total = (long long)B * T * per_row;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const long long bt = i / per_row;
+    const int e = (int)(i - bt * per_row), h = e / per, c = e - h * per;
+    const int b = (int)(bt / T), t = (int)(bt - (long long)b * T);
+    const int pg = t / page_rows, in = t - pg * page_rows;
+    const long long dst = b * c_batch + h * c_head + pg * c_page + (long long)in * D + c * 8;
+    *reinterpret_cast<uint4*>(k_cache + dst) = *reinterpret_cast<const uint4*>(k + b * k_batch + t * k_row + e * 8);
+    *reinterpret_cast<uint4*>(v_cache + dst) = *reinterpret_cast<const uint4*>(v + b * v_batch + t * v_row + e * 8);
+  }
+}
+
 template <int D>
 int launch_partial(const DecodeParams& p, int G, cudaStream_t s) {
   const dim3 grid(p.splits, p.Hkv, p.B);
@@ -549,6 +570,23 @@ extern "C" int b200_kv_append(const void* k_new, const void* v_new, long long kn
       b200host::pdl_enabled() != 0, (const __nv_bfloat16*)k_new, (const __nv_bfloat16*)v_new, kn_batch, vn_batch,
       (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, (const int*)positions, c_batch, c_head, c_page, c_row, page_rows,
       B, Hkv, D));
+}
+
+// Rows 0 .. T-1 of every sequence of head-major paged caches whose rows are D elements apart; k, v: [B, T, Hkv, D] views
+// with dense heads and element strides between rows and sequences.
+extern "C" int b200_kv_write_prompt(const void* k, const void* v, long long k_row, long long k_batch, long long v_row,
+                                    long long v_batch, void* k_cache, void* v_cache, long long c_batch, long long c_head,
+                                    long long c_page, int page_rows, int B, int T, int Hkv, int D, void* stream) {
+  if (B <= 0 || T <= 0 || Hkv <= 0 || D <= 0 || D % 8 || page_rows < 1) return -2;
+  if ((k_row % 8) || (k_batch % 8) || (v_row % 8) || (v_batch % 8) || (c_batch % 8) || (c_head % 8) || (c_page % 8)) return -1;
+  if ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(k_cache) |
+       reinterpret_cast<uintptr_t>(v_cache)) & 15)
+    return -1;
+  const long long blocks = ((long long)B * T * Hkv * (D / 8) + 255) / 256;
+  kv_write_prompt_kernel<<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, k_row, k_batch, v_row, v_batch, (__nv_bfloat16*)k_cache,
+      (__nv_bfloat16*)v_cache, c_batch, c_head, c_page, page_rows, B, T, Hkv, D);
+  return static_cast<int>(cudaGetLastError());
 }
 
 // Splits for the tile-streaming kernel: one wave of resident CTAs (shared memory allows two per SM for GQA groups

@@ -131,3 +131,20 @@ def kv_append_paged(k_new: torch.Tensor, v_new: torch.Tensor, k_pool: torch.Tens
                             v_pool.data_ptr(), positions.data_ptr(), k_pool.stride(0), k_pool.stride(2),
                             k_pool.stride(1), D, k_pool.shape[3], B, Hkv, D, native._stream())
     native._check(rc, "b200_kv_append")
+
+
+def kv_write_prompt_paged(k: torch.Tensor, v: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor) -> None:
+    """Write rows ``0 .. T-1`` of every sequence (``k`` / ``v``: ``[B, T, Hkv, D]`` views with dense heads) into
+    head-major paged caches ``[B, pages, Hkv, page_rows, D]``."""
+
+    lib = native.load()
+    B, T, Hkv, D = k.shape
+    for t in (k, v):
+        if t.dtype != torch.bfloat16 or t.stride(3) != 1 or t.stride(2) != D:
+            raise KernelError("k / v must be bf16 [B,T,Hkv,D] views with heads D elements apart")
+    if v.shape != k.shape or T > k_pool.shape[1] * k_pool.shape[3] or not (k_pool.is_contiguous() and v_pool.is_contiguous()):
+        raise KernelError("the prompt does not fit the paged caches, or they are not contiguous")
+    rc = lib.b200_kv_write_prompt(k.data_ptr(), v.data_ptr(), k.stride(1), k.stride(0) if B > 1 else 0, v.stride(1),
+                                  v.stride(0) if B > 1 else 0, k_pool.data_ptr(), v_pool.data_ptr(), k_pool.stride(0),
+                                  k_pool.stride(2), k_pool.stride(1), k_pool.shape[3], B, T, Hkv, D, native._stream())
+    native._check(rc, "b200_kv_write_prompt")

@@ -92,6 +92,9 @@ def _declare(lib: ctypes.CDLL) -> None:
         c_int, c_int, c_int, c_float, c_float, c_int, c_void_p)
     sig("b200_qknorm_rope_bwd_qk", c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_void_p,
         c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_float, c_int, c_void_p)
+    sig("b200_kv_upper_bound", c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p)
+    sig("b200_kv_write_prompt", c_void_p, c_void_p, c_ll, c_ll, c_ll, c_ll, c_void_p, c_void_p, c_ll, c_ll, c_ll, c_int,
+        c_int, c_int, c_int, c_int, c_void_p)
     sig("b200_swiglu_fwd", c_void_p, c_void_p, c_ll, c_int, c_void_p)
     sig("b200_swiglu_bwd", c_void_p, c_void_p, c_void_p, c_ll, c_int, c_void_p)
     sig("b200_sigmoid_gate_fwd", c_void_p, c_void_p, c_void_p, c_ll, c_void_p)
@@ -640,6 +643,12 @@ def kv_visibility_upper_bound(lo: torch.Tensor, kv_len: int | None = None, q_off
 
     B, S = lo.shape
     n = S if kv_len is None else kv_len
+    if lo.is_cuda and lo.dtype == torch.int32 and lo.numel() > 0 and 0 < n and B <= 65535:
+        lo = lo.contiguous()
+        hi = torch.empty((B, n), dtype=torch.int32, device=lo.device)
+        _check(load().b200_kv_upper_bound(lo.data_ptr(), hi.data_ptr(), B, S, n, int(q_offset), _stream()),
+               "b200_kv_upper_bound")
+        return hi
     k = torch.arange(n, device=lo.device, dtype=lo.dtype).expand(B, n).contiguous()
     return (torch.searchsorted(lo.contiguous(), k, right=True) - 1 + q_offset).to(torch.int32)
 

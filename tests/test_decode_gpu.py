@@ -189,3 +189,43 @@ def test_sampler_kernel_threshold_logprob_and_distribution():
     probs[[0, 1, 4, 7]] = torch.softmax(kept, 0)
     assert float((freq.cpu() - probs).abs().max()) < 0.03, (freq, probs)
     native.check_status()
+
+
+# lengths around a page, one and several sequences, head sizes of the cache kernels; K and V are column ranges of one
+# packed projection
+@pytest.mark.parametrize("T", [2, 127, 128, 129, 300])
+@pytest.mark.parametrize("B,Hkv,D", [(1, 1, 64), (3, 2, 128), (2, 5, 64)])
+def test_prompt_rows_in_pages(T, B, Hkv, D):
+    from research_b200.infer.generation import PagedKVCache
+    from research_b200.ops import native
+
+    hq = 2 * Hkv
+    packed = torch.randn(B, T, (hq + 2 * Hkv) * D, device="cuda").bfloat16()
+    q = packed[..., : hq * D].view(B, T, hq, D)
+    k = packed[..., hq * D:(hq + Hkv) * D].view(B, T, Hkv, D)
+    v = packed[..., (hq + Hkv) * D:].view(B, T, Hkv, D)
+    pos = torch.arange(T, device="cuda", dtype=torch.int32).expand(B, T).contiguous()
+    make = lambda: PagedKVCache(layers=2, batch=B, max_len=T + 5, kv_heads=Hkv, head_dim=D, page_size=128,  # noqa: E731
+                                dtype=torch.bfloat16, device=torch.device("cuda"))
+    told, found = make(), make()
+    with told.prompt():
+        a = told.update_and_attend(1, q, k, v, pos, None)
+    b = found.update_and_attend(1, q, k, v, pos, None)
+    c, _ = native.attn_fwd(q.contiguous(), k.contiguous(), v.contiguous())
+    native.check_status()
+    assert torch.equal(a, b) and torch.equal(a, c.reshape(B, T, -1))
+    for cache in (told, found):
+        assert torch.equal(cache._rows(cache.k, 1, T), k) and torch.equal(cache._rows(cache.v, 1, T), v)
+        assert not cache.k[0].any() and not cache._rows(cache.k, 1, cache.max_len)[:, T:].any()
+    assert not told._from_zero
+
+
+@pytest.mark.parametrize("S,n,off", [(1, 1, 0), (5, 3, 0), (129, 300, 128), (1000, 1000, 0)])
+def test_kv_upper_bound_matches_a_search(S, n, off):
+    from research_b200.ops import native
+
+    g = torch.Generator().manual_seed(S)
+    lo = torch.randint(0, n, (3, S), generator=g, dtype=torch.int32).sort(dim=1).values
+    want = native.kv_visibility_upper_bound(lo, n, off)
+    got = native.kv_visibility_upper_bound(lo.cuda(), n, off)
+    assert got.dtype == torch.int32 and torch.equal(got.cpu(), want)
