@@ -18,6 +18,7 @@ from contextlib import contextmanager
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from research_b200.ops import native
 
@@ -61,6 +62,14 @@ def reference_mode(enabled: bool = True):
 
 def use_native(t: torch.Tensor) -> bool:
     return t.is_cuda and t.dtype == torch.bfloat16 and not _FORCE_REFERENCE
+
+
+def _no_derivatives() -> bool:
+    """True where nothing records or transforms the call: gradients off, no functorch transform, no forward-mode level.
+    The kernels are then called without the autograd function around them (5 to 8 us of host time a call)."""
+
+    return (not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active()
+            and forward_ad._current_level < 0)
 
 
 def _ordered_sums_only() -> bool:
@@ -127,6 +136,9 @@ def linear(x: torch.Tensor, p: torch.Tensor) -> torch.Tensor:
             w = compute_weight(p, x)
             y = native.gemm_skinny(x.reshape(-1, x.shape[-1]), w)
             return y.view(*x.shape[:-1], w.shape[0])
+        if _no_derivatives():
+            w = compute_weight(p, x)
+            return native.gemm(x.reshape(-1, x.shape[-1]), w).view(*x.shape[:-1], w.shape[0])
         return _LinearFn.apply(x, p)
     return F.linear(x, p.to(x.dtype))
 
@@ -167,6 +179,8 @@ def _rmsnorm_ref(x, w, eps):
 
 def rmsnorm(x: torch.Tensor, p: torch.Tensor, eps: float) -> torch.Tensor:
     if use_native(x) and not (_ordered_sums_only() and p.requires_grad and torch.is_grad_enabled()):
+        if _no_derivatives():
+            return native.rmsnorm_fwd(x.contiguous(), p, eps)[0]
         return _RmsNormFn.apply(x, None, p, eps)[0]
     return _rmsnorm_ref(x, p, eps)
 
@@ -175,6 +189,9 @@ def add_rmsnorm(x: torch.Tensor, delta: torch.Tensor, p: torch.Tensor, eps: floa
     """``res = x + delta; y = rmsnorm(res)``; returns ``(y, res)`` from one pass over the data."""
 
     if use_native(x) and not (_ordered_sums_only() and p.requires_grad and torch.is_grad_enabled()):
+        if _no_derivatives():
+            y, _, res = native.rmsnorm_fwd(x.contiguous(), p, eps, delta.contiguous())
+            return y, res
         return _RmsNormFn.apply(x, delta, p, eps)
     res = x + delta
     return _rmsnorm_ref(res, p, eps), res
@@ -229,6 +246,10 @@ def qk_norm_rope(qkv: torch.Tensor, wq, wk, positions: torch.Tensor, hq: int, hk
     """
 
     if use_native(qkv) and not (_ordered_sums_only() and wq is not None and torch.is_grad_enabled()):
+        if _no_derivatives():
+            out = torch.empty(qkv.shape[0], (hq + hkv) * D, dtype=qkv.dtype, device=qkv.device)
+            native.qknorm_rope_fwd_qk(qkv, out, wq, wk, positions, hq, hkv, D, eps, theta, rope)
+            return out
         return _QkNormRopeFn.apply(qkv, wq, wk, positions, hq, hkv, D, eps, theta, rope)
     T = qkv.shape[0]
     q = qkv[:, : hq * D].reshape(T, hq, D)
@@ -328,44 +349,26 @@ class _AttentionBlockFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, wq, wk, positions, lo, hi, B, S, hq, hkv, D, eps, theta, rope, causal, scale):
         T = B * S
-        qk = torch.empty(T, (hq + hkv) * D, dtype=qkv.dtype, device=qkv.device)
-        rq = rk = None
+        rq = None
+        qk = qkv
         if wq is not None or rope:
+            qk = torch.empty(T, (hq + hkv) * D, dtype=qkv.dtype, device=qkv.device)
             rq = native.qknorm_rope_fwd_qk(qkv, qk, wq, wk, positions, hq, hkv, D, eps, theta, rope)
-            q4 = qk[:, : hq * D].view(B, S, hq, D)
-            k4 = qk[:, hq * D:].view(B, S, hkv, D)
-        else:
-            q4 = qkv[:, : hq * D].view(B, S, hq, D)
-            k4 = qkv[:, hq * D:(hq + hkv) * D].view(B, S, hkv, D)
-        v4 = qkv[:, (hq + hkv) * D:].view(B, S, hkv, D)
-        o, lse = native.attn_fwd(q4, k4, v4, causal=causal, lo=lo, scale=scale)
-        ctx.save_for_backward(qkv, qk, o, lse, positions, lo, hi, rq, rk)
+        o, lse = native.attn_fwd_packed(qk, qkv, B, S, hq, hkv, D, causal=causal, lo=lo, scale=scale)
+        ctx.save_for_backward(qkv, qk, o, lse, positions, lo, hi, rq)
         ctx.params = (wq, wk)
         ctx.cfg = (B, S, hq, hkv, D, theta, rope, causal, scale)
-        return o.view(B, S, hq * D)
+        return o
 
     @staticmethod
     def backward(ctx, d_o):
-        qkv, qk, o, lse, positions, lo, hi, rq, rk = ctx.saved_tensors
+        qkv, qk, o, lse, positions, lo, hi, rq = ctx.saved_tensors
         wq, wk = ctx.params
         B, S, hq, hkv, D, theta, rope, causal, scale = ctx.cfg
-        T = B * S
-        transformed = rq is not None or rope
-        if transformed:
-            q4 = qk[:, : hq * D].view(B, S, hq, D)
-            k4 = qk[:, hq * D:].view(B, S, hkv, D)
-        else:
-            q4 = qkv[:, : hq * D].view(B, S, hq, D)
-            k4 = qkv[:, hq * D:(hq + hkv) * D].view(B, S, hkv, D)
-        v4 = qkv[:, (hq + hkv) * D:].view(B, S, hkv, D)
         dqkv = torch.empty_like(qkv)
-        outs = (dqkv[:, : hq * D].view(B, S, hq, D), dqkv[:, hq * D:(hq + hkv) * D].view(B, S, hkv, D),
-                dqkv[:, (hq + hkv) * D:].view(B, S, hkv, D))
-        d_o4 = d_o.reshape(B, S, hq, D)
-        if not d_o4.is_contiguous():
-            d_o4 = d_o4.contiguous()
-        native.attn_bwd(q4, k4, v4, o, d_o4, lse, causal=causal, lo=lo, hi=hi, scale=scale, out=outs)
-        if transformed:  # in place: every (token, head) vector is read and rewritten by one warp
+        native.attn_bwd_packed(qk, qkv, o, d_o.contiguous(), lse, dqkv, B, S, hq, hkv, D, causal=causal, lo=lo, hi=hi,
+                               scale=scale)
+        if rq is not None or rope:  # in place: every (token, head) vector is read and rewritten by one warp
             native.qknorm_rope_bwd_qk(qkv, dqkv, dqkv, wq, wk, positions, rq, None if wq is None else _main_grad(wq),
                                       None if wk is None else _main_grad(wk), hq, hkv, D, theta, rope)
         return (dqkv,) + (None,) * 15
@@ -415,7 +418,7 @@ def swiglu(gu: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` over a fused ``[..., 2I]`` tensor whose first half is the gate."""
 
     if use_native(gu) and (gu.shape[-1] // 2) % 8 == 0:
-        return _SwigluFn.apply(gu)
+        return native.swiglu_fwd(gu.contiguous()) if _no_derivatives() else _SwigluFn.apply(gu)
     inter = gu.shape[-1] // 2
     return F.silu(gu[..., :inter]) * gu[..., inter:]
 
