@@ -8,18 +8,24 @@
 //        S^T = K Q^T,  dP^T = V dO^T,  dV = sum P^T dO,  dS^T = P^T o (dP^T - delta),  dK = scale * sum dS^T Q.
 // Both recompute P from the saved log-sum-exp, so no atomics are needed and results are deterministic.
 //
-// Roles: warp 0 TMA producer (resident tiles once, streamed operands through a 4-slot ring), warp 1 MMA
+// Roles: warp 0 TMA producer (resident tiles once, streamed operands through a 5-slot ring), warp 1 MMA
 // issuer, warps 2-9 element-wise stage: warp w owns TMEM lane quadrant w % 4 and one 64-column half of
 // the 128 x 128 score tile, so two warps share each row.
 //
-// Software pipeline: the score MMA of block n+1 is issued as soon as the element-wise warps have copied
-// S(n) out of tensor memory, so the tensor pipe works on block n+1 while block n's exponentials run.
-// dS goes back to tensor memory as packed bf16 (in place over dP in the dKV kernel, where all 512 columns
-// are taken) and is the A operand of the accumulate MMA straight from there; only P^T of the dKV kernel
-// takes the trip through 128-byte swizzled shared memory.  The streamed operand is consumed a second time
-// as an MN-major B operand from its ring slot (no transposed copy).  Per-query statistics of the dKV
-// kernel (lse, delta of the streamed block) are staged through a small double-buffered shared array one
-// block ahead.
+// Software pipeline: the score MMA of block n+1 is issued as soon as the element-wise warps have copied S(n) out of
+// tensor memory (dQ) or P^T(n) has been consumed (dKV), so the tensor pipe works on block n+1 while block n is in the
+// element-wise stage.  dS goes back to tensor memory as packed bf16 (in place over dP in the dKV kernel, where all 512
+// columns are taken), P^T in place over S^T, and both are the A operand of their accumulate MMA straight from there; the
+// tensor pipe runs in issue order, so the score MMA that overwrites them needs no barrier.  The streamed operand is
+// consumed a second time as an MN-major B operand from its ring slot (no transposed copy).  Per-query statistics of the
+// dKV kernel (lse, delta of the streamed block) are staged through a small double-buffered shared array one block ahead.
+//
+// What bounds it: a block is 3 (dQ) or 4 (dKV) products of 512 clocks and 2 x 64 exponentials a thread pair (1024 clocks
+// of the special-function units).  A tile of the ring is used twice, at both ends of a block, so with four slots the load
+// of block n+2 could only start when block n was finished and its first product waited for it: 2780 and 3700 clocks a
+// block.  P^T in shared memory took the fifth slot's place.  Now 2040 and
+// 2700: 8 x 4096 tokens of 16 / 8 heads of 128, causal, 2010 us at first, 1690 us now (815 TFLOP/s by the count of five
+// products, 1140 by the seven that the two kernels make); one sequence of 16384 3260 -> 2730 us; 777 tokens 53 -> 34 us.
 //
 // Masks as in the forward kernel: query row q sees kv positions [lo[q], q] (causal) or [lo[q], S).
 // `hi` (int32 [B,Skv], non-decreasing) is the kv-side view: the last query position that can see kv k;
@@ -45,20 +51,19 @@ using namespace b200;
 namespace {
 
 constexpr int TILE = 128;
-constexpr int RING = 4;
+constexpr int RING = 5;
 constexpr int EW_WARPS = 8;
-constexpr int NUM_THREADS = 32 * (2 + EW_WARPS);
+constexpr int STAT_WARP = 2 + EW_WARPS;            // dKV: fetches the per-query statistics
+constexpr int NUM_THREADS = 32 * (STAT_WARP + 1);
 constexpr float kLog2e = 1.4426950408889634f;
 
 template <int D>
 struct BwdSmem {
   static constexpr int TILE_BYTES = TILE * D * 2;
-  static constexpr int BUF_BYTES = TILE * TILE * 2;  // P^T staging (dKV), also the epilogue staging
-  static constexpr int X_OFF = 0;                    // two resident tiles
+  static constexpr int X_OFF = 0;                    // two resident tiles; the first is also the epilogue staging
   static constexpr int RING_OFF = X_OFF + 2 * TILE_BYTES;
-  static constexpr int BUF_OFF = RING_OFF + RING * TILE_BYTES;
-  static constexpr int STAT_OFF = BUF_OFF + BUF_BYTES;  // [2][lse2[128], delta[128]] fp32
-  static constexpr int BAR_OFF = STAT_OFF + 2 * 2 * TILE * 4;
+  static constexpr int STAT_OFF = RING_OFF + RING * TILE_BYTES;  // -lse2 [2][128], -delta [3][128], fp32
+  static constexpr int BAR_OFF = STAT_OFF + 5 * TILE * 4;
   static constexpr int TOTAL = BAR_OFF + 256;
 };
 
@@ -71,6 +76,7 @@ struct BwdParams {
   const float* lse;    // [B,Hq,S]
   const float* delta;  // [B,Hq,S]
   int* status;
+  int overlap;         // the dKV kernel is a programmatic dependent of the dQ kernel (see launch_bwd)
   b200ring::RingArgs ring;
 };
 
@@ -95,18 +101,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
     if (threadIdx.x == 0) atomicCAS(p.status, 0, ERR_BAD_ARG);
     return;
   }
+  if (!DKV && p.overlap) pdl_launch_dependents();
   uint64_t* x_full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint64_t* full = x_full + 1;
   uint64_t* empty = full + RING;
-  uint64_t* s_full = empty + RING;     // S(n) is in tensor memory
+  uint64_t* s_full = empty + RING;     // S(n) is in tensor memory (dKV: and its statistics in shared memory)
   uint64_t* dp_full = s_full + 1;      // dP(n) is in tensor memory
-  uint64_t* t1_free = dp_full + 1;     // S(n) has been copied out
-  uint64_t* p_ready = t1_free + 1;     // P^T(n) is in shared memory (dKV)
-  uint64_t* dv_done = p_ready + 1;     // the MMA that read P^T(n) has finished (dKV)
-  uint64_t* ds_ready = dv_done + 1;    // dS(n) is in tensor memory
+  uint64_t* t1_free = dp_full + 1;     // S(n) has been copied out (dQ)
+  uint64_t* p_ready = t1_free + 1;     // P^T(n) is in tensor memory (dKV)
+  uint64_t* ds_ready = p_ready + 1;    // dS(n) is in tensor memory
   uint64_t* acc_done = ds_ready + 1;   // every MMA has finished
-  uint64_t* stat_ready = acc_done + 1; // statistics of block n are in shared memory (dKV)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat_ready + 1);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const AbortCtx ab{abort_flag, p.status};
 
@@ -166,14 +171,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(s_full, 1);
+    mbar_init(s_full, DKV ? 2 : 1);
     mbar_init(dp_full, 1);
     mbar_init(t1_free, EW_WARPS);
     mbar_init(p_ready, EW_WARPS);
-    mbar_init(dv_done, 1);
     mbar_init(ds_ready, EW_WARPS);
     mbar_init(acc_done, 1);
-    mbar_init(stat_ready, EW_WARPS);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -192,7 +195,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
 
   uint8_t* sX1 = smem + L::X_OFF;
   uint8_t* sX2 = sX1 + L::TILE_BYTES;
-  uint8_t* sBuf = smem + L::BUF_OFF;
+  uint8_t* sBuf = sX1;   // epilogue staging: every product has been made by then
 
   if (is_xfer) {
     // ---------------------------------------------------------------- K/V transfer (context parallelism)
@@ -253,22 +256,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
           tc_mma_ss(d_tmem, a0 + off, b0 + off, idesc_t, kk != 0 ? 1u : 0u);
         }
       };
-      // A = P^T in shared memory
-      auto issue_acc_ss = [&](uint32_t d_tmem, const uint8_t* y, bool accumulate) {
-        const uint64_t a0 = make_smem_desc_sw128(smem_u32(sBuf), 16, 1024);
+      // A = packed dS or P^T in tensor memory: 16 K-elements are 8 columns; the two 64-element halves sit 64 columns apart
+      auto issue_acc_ts = [&](uint32_t d_tmem, uint32_t a_tmem, const uint8_t* y, bool accumulate) {
         const uint64_t b0 = make_smem_desc_sw128(smem_u32(y), 16384, 1024);
 #pragma unroll
         for (int kk = 0; kk < TILE / 16; ++kk) {
-          const uint64_t a_off = (uint64_t)(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4);
-          tc_mma_ss(d_tmem, a0 + a_off, b0 + (uint64_t)((kk * 2048) >> 4), idesc_a, (accumulate || kk != 0) ? 1u : 0u);
-        }
-      };
-      // A = packed dS in tensor memory: 16 K-elements are 8 columns; the two 64-element halves sit 64 columns apart
-      auto issue_acc_ts = [&](uint32_t d_tmem, const uint8_t* y, bool accumulate) {
-        const uint64_t b0 = make_smem_desc_sw128(smem_u32(y), 16384, 1024);
-#pragma unroll
-        for (int kk = 0; kk < TILE / 16; ++kk) {
-          tc_mma_ts(d_tmem, tm_DS + (kk >> 2) * 64 + (kk & 3) * 8, b0 + (uint64_t)((kk * 2048) >> 4), idesc_a,
+          tc_mma_ts(d_tmem, a_tmem + (kk >> 2) * 64 + (kk & 3) * 8, b0 + (uint64_t)((kk * 2048) >> 4), idesc_a,
                     (accumulate || kk != 0) ? 1u : 0u);
         }
       };
@@ -289,31 +282,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
         const uint32_t ph = n & 1;
         const bool has_next = n + 1 < n_total;
         const int it_s = 2 * n + 2, it_p = 2 * n + 3;
-        bool s_issued = !has_next;
-        // S(n+1) ahead of everything else when its operands are already there
-        if (has_next && mbar_try_wait(&full[it_s % RING], (it_s / RING) & 1) && mbar_try_wait(t1_free, ph)) {
-          tc_fence_after();
-          issue_t(tm_T1, sX1, ybuf(it_s));
-          tc_commit(s_full);
-          s_issued = true;
-        }
         if (DKV) {
           if (!mbar_wait(p_ready, ph, ab, ERR_WAIT_P_READY)) { ok = false; break; }
           tc_fence_after();
-          issue_acc_ss(tm_A2, ybuf(2 * n + 1), n > 0);  // dV += P^T dO
-          tc_commit(dv_done);
+          issue_acc_ts(tm_A2, tm_T1, ybuf(2 * n + 1), n > 0);  // dV += P^T dO
           tc_commit(&empty[(2 * n + 1) % RING]);
         }
-        if (!s_issued) {
+        if (has_next) {
+          // S(n+1): over P^T(n), after the product that reads it (dKV), or over S(n) once that has been copied out (dQ)
           if (!ring_wait(it_s)) { ok = false; break; }
-          if (!mbar_wait(t1_free, ph, ab, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+          if (!DKV && !mbar_wait(t1_free, ph, ab, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
           tc_fence_after();
           issue_t(tm_T1, sX1, ybuf(it_s));
           tc_commit(s_full);
         }
         if (!mbar_wait(ds_ready, ph, ab, ERR_WAIT_P_READY)) { ok = false; break; }
         tc_fence_after();
-        issue_acc_ts(tm_A1, ybuf(2 * n), n > 0);  // dQ += dS K   or   dK += dS^T Q
+        issue_acc_ts(tm_A1, tm_DS, ybuf(2 * n), n > 0);  // dQ += dS K   or   dK += dS^T Q
         tc_commit(&empty[(2 * n) % RING]);
         if (has_next) {
           // after the accumulate MMA in issue order: in the dKV kernel dP(n+1) overwrites the dS it read
@@ -325,6 +310,40 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
       }
       if (ok) tc_commit(acc_done);
     }
+  } else if (warp == STAT_WARP) {
+    // ---------------------------------------------------------------- statistics of the streamed queries (dKV)
+    // -lse * log2(e) and -delta of the 128 queries of a block, a block ahead of the element-wise warps, which then have
+    // neither global loads nor a barrier among themselves in their loop.  Rows past the end get -inf, which makes P
+    // vanish there.  S(n-1) being complete says that P(n-2) is stored and dS(n-3) too, so two buffers of the one and
+    // three of the other need no barrier of their own.
+    if (DKV && n_total > 0) {
+      float* stats = reinterpret_cast<float*>(smem + L::STAT_OFF);
+      bool ok = true;
+      int blk = 0, g = 0, third = 0;   // of block n: offset in the range of one query head, that head, n % 3
+      for (int n = 0; n < n_total && ok; ++n) {
+        const long long row = ((long long)b * p.Hq + hkv * G + g) * p.S;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int q = (blk_begin + blk) * TILE + i * 32 + lane;
+          v[i] = q < p.S ? -__ldg(p.lse + row + q) * kLog2e : -CUDART_INF_F;
+          v[4 + i] = q < p.S ? -__ldg(p.delta + row + q) : 0.f;
+        }
+        if (++blk == blk_count) {
+          blk = 0;
+          ++g;
+        }
+        if (n >= 1 && !mbar_wait_warp(s_full, (n - 1) & 1, ab, ERR_WAIT_S_READY)) { ok = false; break; }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          stats[(n & 1) * TILE + i * 32 + lane] = v[i];
+          stats[(2 + third) * TILE + i * 32 + lane] = v[4 + i];
+        }
+        third = third == 2 ? 0 : third + 1;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_full);
+      }
+    }
   } else {
     // ---------------------------------------------------------------- element-wise stage + epilogue
     const int quad = warp & 3;
@@ -332,10 +351,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
     const int row = quad * 32 + lane;
     const int g_row = r0 + row;         // this thread's row: local query row (dQ) or kv position (dKV)
     const int q_pos = p.q_off + g_row;  // dQ only: global position of the query row
-    const int t_ew = threadIdx.x - 64;  // 0..255 among the element-wise threads
     const uint32_t lane_sel = static_cast<uint32_t>(quad * 32) << 16;
     const float scale_log2 = p.scale * kLog2e;
-    float* stats = reinterpret_cast<float*>(smem + L::STAT_OFF);
+    const float* stats = reinterpret_cast<const float*>(smem + L::STAT_OFF);
     float lse2_row = 0.f, delta_row = 0.f;
     int lo_row = 0;
     int q_min = 0, q_max = p.S - 1;  // dKV only: local query rows this kv row is visible to
@@ -350,61 +368,56 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
       if (p.causal) q_min = max(0, g_row - p.q_off);
       if (p.hi && g_row < p.Skv) q_max = min(q_max, p.hi[(long long)b * p.Skv + g_row] - p.q_off);
     }
-    // dKV: thread t < 128 fetches lse * log2(e) of query t of block n, thread t >= 128 its delta;
-    // rows past the end get lse = +inf, which makes P exactly zero there.
-    auto load_stat = [&](int n) -> float {
-      const int g = n / blk_count;
-      const int blk = blk_begin + n % blk_count;
-      const int q = blk * TILE + (t_ew & 127);
-      const long long idx = ((long long)b * p.Hq + hkv * G + g) * p.S + q;
-      if (t_ew < 128) return q < p.S ? __ldg(p.lse + idx) * kLog2e : CUDART_INF_F;
-      return q < p.S ? __ldg(p.delta + idx) : 0.f;
-    };
+    const uint64_t scale2 = f2_pack(scale_log2, scale_log2);
+    const uint64_t minus_lse = f2_pack(-lse2_row, -lse2_row), minus_delta = f2_pack(-delta_row, -delta_row);
     bool ok = n_total > 0;
-    if (DKV && ok) {
-      stats[t_ew] = load_stat(0);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(stat_ready);
-    }
-    for (int n = 0; n < n_total && ok; ++n) {
+    int blk = blk_begin, third = 0;   // of block n, and n % 3
+    for (int n = 0; n < n_total && ok; ++n, blk = blk + 1 == blk_begin + blk_count ? blk_begin : blk + 1) {
       const uint32_t ph = n & 1;
-      const int blk = blk_begin + (DKV ? n % blk_count : n);
-      float stat_next = 0.f;
-      if (DKV && n + 1 < n_total) stat_next = load_stat(n + 1);
-      const float* st = stats + (n & 1) * 256 + half * 64;  // lse2 of this warp's 64 columns; delta 128 floats on
-      if (DKV && !mbar_wait_warp(stat_ready, ph, ab, ERR_WAIT_S_READY)) { ok = false; break; }
+      // dKV: statistics of this warp's 64 columns
+      const float* st_lse = stats + (n & 1) * TILE + half * 64;
+      const float* st_delta = stats + (2 + third) * TILE + half * 64;
+      third = third == 2 ? 0 : third + 1;
       if (!mbar_wait_warp(s_full, ph, ab, ERR_WAIT_S_READY)) { ok = false; break; }
       tc_fence_after();
+      // P of this thread's 64 columns, in pairs, every fourth pair on the FMA pipes: the special-function unit alone
+      // would take 1024 clocks a block (16384 tokens 2816 us without, 2765 us with; half of the pairs 2834 us).
       float pv[64];
       {
         uint32_t ra[32], rb[32];
         tmem_ld_32x32b_x32(tm_T1 + lane_sel + half * 64, ra);
         tmem_ld_32x32b_x32(tm_T1 + lane_sel + half * 64 + 32, rb);
         tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(t1_free);
         if (!DKV) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            pv[i] = ex2_approx(fmaf(__uint_as_float(ra[i]), scale_log2, -lse2_row));
-            pv[32 + i] = ex2_approx(fmaf(__uint_as_float(rb[i]), scale_log2, -lse2_row));
-          }
-        } else {
-#pragma unroll
-          for (int i4 = 0; i4 < 8; ++i4) {
-            const float4 la = *reinterpret_cast<const float4*>(st + 4 * i4);
-            const float4 lb = *reinterpret_cast<const float4*>(st + 32 + 4 * i4);
-            pv[4 * i4 + 0] = ex2_approx(fmaf(__uint_as_float(ra[4 * i4 + 0]), scale_log2, -la.x));
-            pv[4 * i4 + 1] = ex2_approx(fmaf(__uint_as_float(ra[4 * i4 + 1]), scale_log2, -la.y));
-            pv[4 * i4 + 2] = ex2_approx(fmaf(__uint_as_float(ra[4 * i4 + 2]), scale_log2, -la.z));
-            pv[4 * i4 + 3] = ex2_approx(fmaf(__uint_as_float(ra[4 * i4 + 3]), scale_log2, -la.w));
-            pv[32 + 4 * i4 + 0] = ex2_approx(fmaf(__uint_as_float(rb[4 * i4 + 0]), scale_log2, -lb.x));
-            pv[32 + 4 * i4 + 1] = ex2_approx(fmaf(__uint_as_float(rb[4 * i4 + 1]), scale_log2, -lb.y));
-            pv[32 + 4 * i4 + 2] = ex2_approx(fmaf(__uint_as_float(rb[4 * i4 + 2]), scale_log2, -lb.z));
-            pv[32 + 4 * i4 + 3] = ex2_approx(fmaf(__uint_as_float(rb[4 * i4 + 3]), scale_log2, -lb.w));
-          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(t1_free);
         }
+        auto probs = [&](const uint32_t (&r)[32], int base) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            uint64_t la = minus_lse, lb = minus_lse;
+            if (DKV) {
+              const float4 l = *reinterpret_cast<const float4*>(st_lse + base + i);
+              la = f2_pack(l.x, l.y);
+              lb = f2_pack(l.z, l.w);
+            }
+            const uint64_t xa = f2_fma(f2_pack(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), scale2, la);
+            const uint64_t xb = f2_fma(f2_pack(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), scale2, lb);
+            f2_unpack(xa, pv[base + i], pv[base + i + 1]);
+            pv[base + i] = ex2_approx(pv[base + i]);
+            pv[base + i + 1] = ex2_approx(pv[base + i + 1]);
+            if ((i / 4) & 1) {
+              f2_unpack(f2_ex2(xb), pv[base + i + 2], pv[base + i + 3]);
+            } else {
+              f2_unpack(xb, pv[base + i + 2], pv[base + i + 3]);
+              pv[base + i + 2] = ex2_approx(pv[base + i + 2]);
+              pv[base + i + 3] = ex2_approx(pv[base + i + 3]);
+            }
+          }
+        };
+        probs(ra, 0);
+        probs(rb, 32);
       }
       const int c0 = blk * TILE + half * 64;  // first column of this warp: kv position (dQ) or local query row (dKV)
       if (!DKV) {
@@ -423,17 +436,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
           for (int i = 0; i < 64; ++i)
             if (c0 + i < q_min || c0 + i > q_max) pv[i] = 0.f;
         }
-        if (n > 0 && !mbar_wait_warp(dv_done, ph ^ 1, ab, ERR_WAIT_O_READY)) { ok = false; break; }
+        uint32_t packed[32];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          uint4 v;
-          v.x = pack_bf16x2(pv[8 * k + 0], pv[8 * k + 1]);
-          v.y = pack_bf16x2(pv[8 * k + 2], pv[8 * k + 3]);
-          v.z = pack_bf16x2(pv[8 * k + 4], pv[8 * k + 5]);
-          v.w = pack_bf16x2(pv[8 * k + 6], pv[8 * k + 7]);
-          *reinterpret_cast<uint4*>(sBuf + half * 16384 + sw128_offset(row, k)) = v;
-        }
-        fence_proxy_async_smem();
+        for (int k = 0; k < 32; ++k) packed[k] = pack_bf16x2(pv[2 * k], pv[2 * k + 1]);
+        tmem_st_32x32b_x32(tm_T1 + lane_sel + half * 64, packed);   // over this warp's own scores
+        tmem_st_wait();
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(p_ready);
       }
@@ -444,40 +452,32 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
         tmem_ld_32x32b_x32(tm_T2 + lane_sel + half * 64, ra);
         tmem_ld_32x32b_x32(tm_T2 + lane_sel + half * 64 + 32, rb);
         tmem_ld_wait();
-        if (!DKV) {
+        auto dscores = [&](const uint32_t (&r)[32], int base) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            packed[i] = pack_bf16x2(pv[2 * i] * (__uint_as_float(ra[2 * i]) - delta_row),
-                                    pv[2 * i + 1] * (__uint_as_float(ra[2 * i + 1]) - delta_row));
-            packed[16 + i] = pack_bf16x2(pv[32 + 2 * i] * (__uint_as_float(rb[2 * i]) - delta_row),
-                                         pv[32 + 2 * i + 1] * (__uint_as_float(rb[2 * i + 1]) - delta_row));
+          for (int i = 0; i < 32; i += 4) {
+            uint64_t da = minus_delta, db = minus_delta;
+            if (DKV) {
+              const float4 d = *reinterpret_cast<const float4*>(st_delta + base + i);
+              da = f2_pack(d.x, d.y);
+              db = f2_pack(d.z, d.w);
+            }
+            float x, y;
+            f2_unpack(f2_mul(f2_pack(pv[base + i], pv[base + i + 1]),
+                             f2_add(f2_pack(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), da)), x, y);
+            packed[(base + i) / 2] = pack_bf16x2(x, y);
+            f2_unpack(f2_mul(f2_pack(pv[base + i + 2], pv[base + i + 3]),
+                             f2_add(f2_pack(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), db)), x, y);
+            packed[(base + i) / 2 + 1] = pack_bf16x2(x, y);
           }
-        } else {
-#pragma unroll
-          for (int i4 = 0; i4 < 8; ++i4) {
-            const float4 da = *reinterpret_cast<const float4*>(st + 128 + 4 * i4);
-            const float4 db = *reinterpret_cast<const float4*>(st + 128 + 32 + 4 * i4);
-            packed[2 * i4] = pack_bf16x2(pv[4 * i4] * (__uint_as_float(ra[4 * i4]) - da.x),
-                                         pv[4 * i4 + 1] * (__uint_as_float(ra[4 * i4 + 1]) - da.y));
-            packed[2 * i4 + 1] = pack_bf16x2(pv[4 * i4 + 2] * (__uint_as_float(ra[4 * i4 + 2]) - da.z),
-                                             pv[4 * i4 + 3] * (__uint_as_float(ra[4 * i4 + 3]) - da.w));
-            packed[16 + 2 * i4] = pack_bf16x2(pv[32 + 4 * i4] * (__uint_as_float(rb[4 * i4]) - db.x),
-                                              pv[32 + 4 * i4 + 1] * (__uint_as_float(rb[4 * i4 + 1]) - db.y));
-            packed[16 + 2 * i4 + 1] = pack_bf16x2(pv[32 + 4 * i4 + 2] * (__uint_as_float(rb[4 * i4 + 2]) - db.z),
-                                                  pv[32 + 4 * i4 + 3] * (__uint_as_float(rb[4 * i4 + 3]) - db.w));
-          }
-        }
+        };
+        dscores(ra, 0);
+        dscores(rb, 32);
         tmem_st_32x32b_x32(tm_DS + lane_sel + half * 64, packed);
         tmem_st_wait();
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_ready);
-      if (DKV && n + 1 < n_total) {
-        stats[((n + 1) & 1) * 256 + t_ew] = stat_next;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(stat_ready);
-      }
     }
     // ---- epilogue: accumulators -> bf16 -> global.  Warp (quad, half) owns rows quad*32.. and the
     //      64-column box `half` of the D columns (for D = 64 only half 0 has columns).  The softmax scale
@@ -543,6 +543,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  if (DKV && p.overlap) pdl_wait();   // what follows in the stream sees the dQ kernel's results as well
 }
 
 // delta[b,h,s] = sum_d dO[b,s,h,d] * O[b,s,h,d]; D / 8 lanes per (b,s,h), so a warp covers 32 / (D / 8) heads at once
@@ -593,8 +594,12 @@ int launch_bwd(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& 
   if (int rc = b200host::ensure_dynamic_smem(kern, smem_bytes, configured)) return rc;
   const int tiles = ((DKV ? p.Skv : p.S) + TILE - 1) / TILE;
   const int grid = tiles * (DKV ? p.Hkv : p.Hq) * p.B + ((!DKV && p.ring.enabled) ? p.ring.n_transfer : 0);
-  kern<<<grid, NUM_THREADS, smem_bytes, stream>>>(x1, x2, y1, y2, o1, o2, owners, p);
-  return static_cast<int>(cudaGetLastError());
+  // The two kernels share their inputs and write different tensors, so the dKV kernel need not wait for the dQ kernel: as
+  // a programmatic dependent it takes the SMs that the last wave of the dQ kernel leaves free, and waits for its end
+  // only before it ends itself.  delta is complete by then, because the dQ kernel is launched the ordinary way.  Not
+  // with the exchange of context parallelism, where the dQ kernel stages what the dKV kernel reads.
+  return static_cast<int>(b200host::launch_kernel(kern, dim3(grid), dim3(NUM_THREADS), smem_bytes, stream,
+                                                  DKV && p.overlap, x1, x2, y1, y2, o1, o2, owners, p));
 }
 
 }  // namespace
@@ -663,6 +668,7 @@ static int attn_bwd_impl(const void* q, const void* k, const void* v, const void
     tdV = tdQ;
   }
   const OwnerMaps& om = ring ? owner_maps : no_owners;
+  p.overlap = !ring && pdl_enabled();
   if (D == 128) {
     if ((rc = launch_bwd<128, false>(tQ, tdO, tK, tV, tdQ, tdQ, om, p, s))) return rc;
     return launch_bwd<128, true>(tK, tV, tQ, tdO, tdK, tdV, om, p, s);
