@@ -1393,13 +1393,3 @@ extern "C" int b200_cast_f32_bf16(const void* x, void* y, long long n, float sca
   cast_f32_bf16_kernel<<<grid_for(n, 256, 8), 256, 0, STREAM(stream)>>>((const float*)x, (__nv_bfloat16*)y, n, scale);
   return LAST_ERR();
 }
-
-// ws: fp32 [n] holding split-K sums (zeroed again on return), out: bf16 [n]; n % 4 == 0, both 16-byte aligned.
-extern "C" int b200_splitk_finish(void* ws, void* out, long long n, void* stream) {
-  if (n <= 0 || n % 4) return -2;
-  const long long n4 = n / 4;
-  long long blocks = (n4 + 255) / 256;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  return static_cast<int>(b200host::launch_kernel(splitk_finish_kernel, dim3((int)blocks), dim3(256), 0, STREAM(stream),
-                                                  b200host::pdl_enabled() != 0, (float*)ws, (__nv_bfloat16*)out, n4));
-}

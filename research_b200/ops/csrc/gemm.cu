@@ -61,17 +61,6 @@ struct GemmParams {
   const int* k_range;
   // Split-K: the batch index selects a K slice of A and B, and every slice adds into the same C (z = 0).
   int c_shared;
-  // Split-K with the finishing pass inside the kernel (fp32 C is a workspace that is zero between launches): the CTA
-  // that adds the last slice of an output tile converts the tile's sums to bf16 into fin_out and clears the
-  // workspace behind it.  fin_count: one zeroed counter per output tile, left zero.
-  const float* fin_ws_ptr;
-  __nv_bfloat16* fin_out;
-  long long fin_ld_ws, fin_ld_out;
-  unsigned int* fin_count;
-  int fin_splits;
-  // Programmatic dependent launch (skinny split-K products of a decode step): the weight tiles of the first stages
-  // are requested before the wait for the predecessor, only the activation tiles and the output come after it.
-  int pdl;
   // SYM: C = alpha * acc + beta * G + gamma * I, written with its transpose; G (nullptr: none) and C share their strides.
   const __nv_bfloat16* sym_g;
   __nv_bfloat16* sym_c;
@@ -96,15 +85,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
-  if (p.pdl) pdl_launch_dependents();   // the successor may take its place on the SMs; it waits for this grid itself
-
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint64_t* empty = full + STAGES;
   uint64_t* tfull = empty + STAGES;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile unsigned int* fin_prev = reinterpret_cast<volatile unsigned int*>(tmem_slot + 2);
   const AbortCtx ab{abort_flag, p.status};
 
   const int warp = warp_uniform(threadIdx.x >> 5);
@@ -190,25 +176,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           for (int j = 0; j < BN / 64; ++j) tma_load_3d(sB + j * 8192, &tmB, bar, n0 + j * 64, kb * BK, zB);
         }
       };
-      // Dependent launch: B (the weights) does not depend on the predecessor, so the B tiles of the first tile's
-      // first stages are on their way before this CTA waits for it; A follows after the wait.
-      uint32_t b_ahead = 0;
-      if (p.pdl) {
-        if ((int)blockIdx.x < total_tiles) {
-          int b, m0, n0, bB, zAC, kb0, kb1;
-          tile_coords(blockIdx.x, b, m0, n0);
-          if (tile_extent(b, m0, bB, zAC, kb0, kb1)) {
-            const int zB = (p.k_range || p.c_shared) ? 0 : bB;
-            const int k_off = p.c_shared ? b * k_blocks : 0;
-            for (int kb = kb0 + k_off; kb < kb1 + k_off && b_ahead < (uint32_t)STAGES; ++kb, ++b_ahead) {
-              uint8_t* sB = smem + b_ahead * L::STAGE_BYTES + A_TILE_BYTES;
-              mbar_expect_tx(&full[b_ahead], L::STAGE_BYTES);
-              load_b(sB, &full[b_ahead], kb, n0, zB);
-            }
-          }
-        }
-        pdl_wait();
-      }
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         int b, m0, n0, bB, zAC, kb0, kb1;
         tile_coords(t, b, m0, n0);
@@ -219,18 +186,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int kb = kb0 + k_off; kb < kb1 + k_off; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          const bool b_requested = it < b_ahead;   // expect_tx and the B tile of this stage went out before the wait
-          if (!b_requested && !mbar_wait(&empty[s], ph ^ 1, ab, ERR_WAIT_EMPTY)) { ok = false; break; }
+          if (!mbar_wait(&empty[s], ph ^ 1, ab, ERR_WAIT_EMPTY)) { ok = false; break; }
           uint8_t* sA = smem + s * L::STAGE_BYTES;
           uint8_t* sB = sA + A_TILE_BYTES;
-          if (!b_requested) mbar_expect_tx(&full[s], L::STAGE_BYTES);
+          mbar_expect_tx(&full[s], L::STAGE_BYTES);
           if (!A_MN) {
             tma_load_3d(sA, &tmA, &full[s], kb * BK, m0, zA);
           } else {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j) tma_load_3d(sA + j * 8192, &tmA, &full[s], m0 + j * 64, kb * BK, zA);
           }
-          if (!b_requested) load_b(sB, &full[s], kb, n0, zB);
+          load_b(sB, &full[s], kb, n0, zB);
         }
       }
       if (!ok) {
@@ -280,7 +246,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint32_t tile_iter = 0;
     uint32_t box_iter = 0;
     bool ok = true;
-    if (p.pdl) pdl_wait();   // C (and the workspace behind it) belongs to the predecessor until it has completed
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       int b, m0, n0, bB, zAC, kb0, kb1;
       tile_coords(t, b, m0, n0);
@@ -383,38 +348,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
-      if (OUT_F32 && p.fin_out) {
-        // split-K with the finishing pass fused: when this CTA's adds of the tile are in memory, count the slice;
-        // the CTA that counts the last one converts the tile and clears the workspace
-        float* ws = reinterpret_cast<float*>(const_cast<void*>(static_cast<const void*>(p.fin_ws_ptr)));
-        if (lane == 0) {
-          tma_wait_group<0>();
-          fence_proxy_async_all();
-          __threadfence();
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");   // the four epilogue warps
-        const int tile_id = (m0 / BM) * ((p.N + BN - 1) / BN) + n0 / BN;
-        if (warp == 2 && lane == 0) *fin_prev = atomicAdd(&p.fin_count[tile_id], 1u);
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (*fin_prev == (unsigned int)p.fin_splits - 1u) {
-          __threadfence();
-          const int tid = (int)threadIdx.x - 64;          // 0..127 among the epilogue threads
-          const int rows = min(BM, p.M - m0);
-          const int vec_per_row = min(BN, p.N - n0) >> 2;
-          for (int i = tid; i < rows * vec_per_row; i += EPI_WARPS * 32) {
-            const int r = i / vec_per_row, c = (i - r * vec_per_row) << 2;
-            float4* src = reinterpret_cast<float4*>(ws + (long long)(m0 + r) * p.fin_ld_ws + n0 + c);
-            const float4 v = __ldcg(src);
-            uint2 o;
-            o.x = pack_bf16x2(v.x, v.y);
-            o.y = pack_bf16x2(v.z, v.w);
-            *reinterpret_cast<uint2*>(p.fin_out + (long long)(m0 + r) * p.fin_ld_out + n0 + c) = o;
-            __stcg(src, make_float4(0.f, 0.f, 0.f, 0.f));
-          }
-          if (tid == 0) p.fin_count[tile_id] = 0u;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");   // fin_prev may be rewritten for the next tile
-      }
     }
     if (lane == 0) tma_wait_group<0>();
   }
@@ -437,8 +370,6 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
   constexpr int smem_bytes = L::TOTAL + 1024;
   static bool configured[b200host::kMaxDevices] = {};   // per kernel instantiation and device
   if (int rc = b200host::ensure_dynamic_smem(kern, smem_bytes, configured)) return rc;
-  if (p.pdl) return static_cast<int>(b200host::launch_kernel(kern, dim3(grid), dim3(NUM_THREADS), smem_bytes, stream, true,
-                                                             tmA, tmB, tmC, p));
   kern<<<grid, NUM_THREADS, smem_bytes, stream>>>(tmA, tmB, tmC, p);
   return static_cast<int>(cudaGetLastError());
 }
@@ -469,7 +400,6 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
                      int batch_c, long long lda, long long ldb, long long ldc, long long stride_a, long long stride_b,
                      long long stride_c, int a_mn, int b_mn, int out_f32, int accumulate, int bn_hint,
                      const int* tile_group, const int* k_range, int* status, void* stream, int c_shared = 0,
-                     void* fin_out = nullptr, long long fin_ld_out = 0, void* fin_count = nullptr, int pdl = 0,
                      int k_total = 0);
 
 extern "C" int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int batch, long long lda,
@@ -478,29 +408,6 @@ extern "C" int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int 
                               int* status, void* stream) {
   return gemm_impl(A, B, C, M, N, K, batch, batch, batch, batch, lda, ldb, ldc, stride_a, stride_b, stride_c, a_mn,
                    b_mn, out_f32, accumulate, bn_hint, nullptr, nullptr, status, stream);
-}
-
-// Split-K product for skinny problems (few rows, e.g. one decode token per sequence): C[M,N] (fp32, zeroed by the
-// caller) += A[:, slice] * B[:, slice]^T for `splits` equal K slices, one CTA tile per (N tile, slice), so that a
-// weight matrix is streamed by many SMs at once.  K must be a multiple of 64 * splits.
-extern "C" int b200_gemm_bf16_splitk(const void* A, const void* B, void* C, int M, int N, int K, int splits,
-                                     long long lda, long long ldb, long long ldc, int* status, void* stream) {
-  if (splits < 1 || K % (64 * splits)) return b200host::RC_BAD_SHAPE;
-  const int kc = K / splits;
-  return gemm_impl(A, B, C, M, N, kc, splits, 1, 1, 1, lda, ldb, ldc, 0, 0, 0, 0, 0, 1, 1, 0, nullptr, nullptr, status,
-                   stream, 1, nullptr, 0, nullptr, b200host::pdl_enabled());
-}
-
-// The same with the finishing pass inside the kernel: `ws` is an fp32 [M, N] workspace (row stride ldws) that is zero
-// on entry and zero again on exit, `out` receives the bf16 result (row stride ldo), `counters` holds one zeroed
-// uint32 per 128 x BN output tile (left zero).  N, ldws and ldo must be multiples of 4.
-extern "C" int b200_gemm_bf16_splitk_fused(const void* A, const void* B, void* ws, void* out, void* counters, int M,
-                                           int N, int K, int splits, long long lda, long long ldb, long long ldws,
-                                           long long ldo, int* status, void* stream) {
-  if (splits < 1 || K % (64 * splits) || !out || !counters) return b200host::RC_BAD_SHAPE;
-  const int kc = K / splits;
-  return gemm_impl(A, B, ws, M, N, kc, splits, 1, 1, 1, lda, ldb, ldws, 0, 0, 0, 0, 0, 1, 1, 0, nullptr, nullptr,
-                   status, stream, 1, out, ldo, counters, b200host::pdl_enabled());
 }
 
 // Split-K for any operand layout with an fp32 output that is accumulated into (weight gradients: the contraction
@@ -514,7 +421,7 @@ extern "C" int b200_gemm_bf16_splitk_acc(const void* A, const void* B, void* C, 
   const int per = (blocks + splits - 1) / splits;
   splits = (blocks + per - 1) / per;   // no slice is empty
   return gemm_impl(A, B, C, M, N, per * BK, splits, 1, 1, 1, lda, ldb, ldc, 0, 0, 0, a_mn, b_mn, 1, 1, 0, nullptr,
-                   nullptr, status, stream, 1, nullptr, 0, nullptr, 0, K);
+                   nullptr, status, stream, 1, K);
 }
 
 // C[b] = alpha * A[b] A[b]^T + beta * G[b] + gamma * I for a stack of matrices, each C[b] a symmetric d x d matrix of
@@ -580,8 +487,7 @@ extern "C" int b200_gemm_bf16_grouped_k(const void* A, const void* B, void* C, i
 static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K, int batch, int batch_a, int batch_b,
                      int batch_c, long long lda, long long ldb, long long ldc, long long stride_a, long long stride_b,
                      long long stride_c, int a_mn, int b_mn, int out_f32, int accumulate, int bn_hint,
-                     const int* tile_group, const int* k_range, int* status, void* stream, int c_shared, void* fin_out,
-                     long long fin_ld_out, void* fin_count, int pdl, int k_total) {
+                     const int* tile_group, const int* k_range, int* status, void* stream, int c_shared, int k_total) {
   using namespace b200host;
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return RC_BAD_SHAPE;
   const int BN = (bn_hint == 128 || bn_hint == 256) ? bn_hint : (N > 128 ? 256 : 128);
@@ -608,16 +514,6 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
   if (rc) return rc;
 
   GemmParams p{M, N, K, batch, accumulate, status, tile_group, k_range, c_shared};
-  p.fin_ws_ptr = fin_out ? static_cast<const float*>(C) : nullptr;
-  p.fin_out = static_cast<__nv_bfloat16*>(fin_out);
-  p.fin_ld_ws = ldc;
-  p.fin_ld_out = fin_ld_out;
-  p.fin_count = static_cast<unsigned int*>(fin_count);
-  p.fin_splits = batch;
-  p.pdl = pdl;
-  if (fin_out && (!c_shared || !out_f32 || !accumulate || !fin_count || (N & 3) || (ldc & 3) || (fin_ld_out & 3) ||
-                  (reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(fin_out) & 7)))
-    return RC_BAD_SHAPE;
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * batch;
   const int grid = tiles < sm_count() ? tiles : sm_count();
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);

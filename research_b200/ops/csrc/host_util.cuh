@@ -118,6 +118,26 @@ inline int make_map_3d(CUtensorMap* out, CUtensorMapDataType dt, const void* bas
   return RC_OK;
 }
 
+// Rank-2 row-major tensor [d1][d0] with byte stride s1; box {b0, b1}.
+inline int make_map_2d(CUtensorMap* out, CUtensorMapDataType dt, const void* base, uint64_t d0, uint64_t d1,
+                       uint64_t s1_bytes, uint32_t b0, uint32_t b1, CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_128B) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return RC_NO_DRIVER_ENTRY;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (s1_bytes & 15)) return RC_BAD_ALIGNMENT;
+  cuuint64_t dims[2] = {d0, d1};
+  cuuint64_t strides[1] = {s1_bytes};
+  cuuint32_t box[2] = {b0, b1};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    fprintf(stderr, "research_b200: cuTensorMapEncodeTiled(2d) failed (%d) dims=(%llu,%llu) stride=%llu box=(%u,%u)\n", (int)r,
+            (unsigned long long)d0, (unsigned long long)d1, (unsigned long long)s1_bytes, b0, b1);
+    return RC_TENSORMAP_FAILED;
+  }
+  return RC_OK;
+}
+
 // Rank-4 tensor [d3][d2][d1][d0] with byte strides s1 <= s2 <= s3 (each a multiple of the one before,
 // which is why attention orders its dims as head_dim, head, token, batch); box {b0, b1, b2, 1}.
 inline int make_map_4d(CUtensorMap* out, CUtensorMapDataType dt, const void* base, uint64_t d0, uint64_t d1,

@@ -128,10 +128,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         c_float, c_float, c_float, c_void_p)
     sig("b200_gemm_bf16_splitk_acc", c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_int,
         c_int, c_void_p, c_void_p)
-    sig("b200_gemm_bf16_splitk", c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_void_p,
-        c_void_p)
-    sig("b200_gemm_bf16_splitk_fused", c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll,
-        c_ll, c_ll, c_ll, c_void_p, c_void_p)
+    sig("b200_gemm_skinny", c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_void_p, c_void_p)
     sig("b200_sample_topk", c_void_p, c_ll, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p)
     sig("b200_decode_attn_splits", c_int, c_int, c_int, c_int)
     sig("b200_decode_attn", c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
@@ -139,7 +136,6 @@ def _declare(lib: ctypes.CDLL) -> None:
     sig("b200_decode_attn_paged", c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
         c_int, c_int, c_int, c_ll, c_ll, c_ll, c_int, c_float, c_int, c_ll, c_void_p, c_void_p)
     sig("b200_decode_attn_paged_splits", c_int, c_int, c_int, c_int)
-    sig("b200_splitk_finish", c_void_p, c_void_p, c_ll, c_void_p)
     sig("b200_kv_append", c_void_p, c_void_p, c_ll, c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_ll, c_ll, c_ll, c_int,
         c_int, c_int, c_int, c_void_p)
     sig("b200_attn_fwd", c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -350,92 +346,41 @@ def gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, grad: torch.Tensor) -> None:
 
 @functools.lru_cache(maxsize=4096)
 def splitk_factor(n: int, k: int, sms: int = 148) -> int:
-    """How many K slices a skinny ``[rows, k] x [n, k]^T`` product should be cut into so that about one CTA per SM
-    streams the weight (its four-stage ring keeps enough bytes in flight; more slices only add reduce traffic:
-    measured 39 us against 45 us per decoder layer with two CTAs per SM): a divisor of ``k / 64`` that leaves
-    slices of at least 128."""
+    """Slices of K (1, 2, 4 or 8 CTAs of a cluster) for a skinny ``[rows, k] x [n, k]^T`` product: the count of least
+    estimated time, the larger of what the busiest SM streams (0.27 us per 16 KB block of a 128-row tile) and of the
+    whole matrix at 6.3 TB/s, plus the exchange of partial sums.  Slices are at least two blocks.  Measured with 32
+    rows: 4096 x 2048 1 / 2 / 4 / 8 slices 7.8 / 6.8 / 6.4 / 7.0 us, 2048 x 5632 16.4 / 10.0 / 8.3 / 8.0 us, 11264 x 2048
+    10.9 / 12.0 / 11.2 / 16.6 us, 6144 x 4096 13.6 / 11.8 / 12.4 / 12.7 us, 50304 x 2048 34 / 41 / 48 / 65 us."""
 
-    tiles = (n + 255) // 256
-    kblocks = k // 64
-    best = 1
-    for d in range(1, kblocks + 1):
-        if kblocks % d or k // d < 128 or tiles * d > sms:
-            continue
-        best = d
+    tiles, blocks = (n + 127) // 128, k // 64
+    best, best_cost = 1, float("inf")
+    for s, exchange in ((1, 0.0), (2, 1.1), (4, 1.6), (8, 3.0)):
+        if s > 1 and blocks < 2 * s:
+            break
+        cost = max(-(-tiles * s // sms) * -(-blocks // s) * 0.27, n * k * 2 / 6.3e6) + exchange
+        if cost < best_cost:
+            best, best_cost = s, cost
     return best
 
 
 def gemm_skinny(a: torch.Tensor, b: torch.Tensor, fused_finish: bool | None = None) -> torch.Tensor:
-    """``a [rows, K] @ b [N, K]^T`` for a handful of rows (decode): split-K so that the whole device streams ``b``.
-    Returns bf16 ``[rows, N]``.  ``fused_finish``: let the CTA that adds the last slice of a tile convert it inside the
-    product (default: ``RESEARCH_B200_SPLITK_FUSED``, off: inside a CUDA graph the separate 3 us finishing kernel
-    measured cheaper than the counters, fences and barriers that the fused form adds to every CTA)."""
+    """``a [rows, K] @ b [N, K]^T`` for a handful of rows (decode): K is cut over the CTAs of a cluster so that the whole
+    device streams ``b``, and the cluster adds up its partial sums itself.  Returns bf16 ``[rows, N]``.
+    ``fused_finish`` is accepted and has no effect (there is no finishing pass to place)."""
 
-    lib = load()
+    lib = _lib or load()
     rows, K = a.shape
     N = b.shape[0]
-    if K % 64 or a.stride(1) != 1 or b.stride(1) != 1:
+    if K % 64 or rows > 128 or a.stride(1) != 1 or b.stride(1) != 1:
         return gemm(a, b, trans_b=True)
-    splits = splitk_factor(N, K)
-    if splits == 1:
-        return gemm(a, b, trans_b=True)
-    if N % 4:
-        c = torch.zeros((rows, N), dtype=torch.float32, device=a.device)
-        rc = lib.b200_gemm_bf16_splitk(a.data_ptr(), b.data_ptr(), c.data_ptr(), rows, N, K, splits, a.stride(0),
-                                       b.stride(0), c.stride(0), status_word(a.device).data_ptr(), _stream())
-        _check(rc, "b200_gemm_bf16_splitk")
-        return c.to(torch.bfloat16)
-    # the slices add into a persistent fp32 workspace that is zero between calls; a finishing pass (a small kernel,
-    # or the CTA that adds the last slice of a tile) converts the sums to bf16 and clears the workspace behind it,
-    # so a decode step runs no fill and no cast per linear
-    ws = _splitk_workspace(rows * N, a.device)
+    if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or b.shape[1] != K:
+        raise KernelError(f"gemm_skinny expects bf16 operands with one inner dimension, got {tuple(a.shape)} {a.dtype} "
+                          f"and {tuple(b.shape)} {b.dtype}")
     out = torch.empty((rows, N), dtype=torch.bfloat16, device=a.device)
-    try:
-        if rows <= 128 and (fused_finish if fused_finish is not None
-                            else os.environ.get("RESEARCH_B200_SPLITK_FUSED", "0") == "1"):
-            counters = _splitk_counters(a.device)
-            rc = lib.b200_gemm_bf16_splitk_fused(a.data_ptr(), b.data_ptr(), ws.data_ptr(), out.data_ptr(),
-                                                 counters.data_ptr(), rows, N, K, splits, a.stride(0), b.stride(0), N,
-                                                 N, status_word(a.device).data_ptr(), _stream())
-            _check(rc, "b200_gemm_bf16_splitk_fused")
-            return out
-        rc = lib.b200_gemm_bf16_splitk(a.data_ptr(), b.data_ptr(), ws.data_ptr(), rows, N, K, splits, a.stride(0),
-                                       b.stride(0), N, status_word(a.device).data_ptr(), _stream())
-        _check(rc, "b200_gemm_bf16_splitk")
-        _check(lib.b200_splitk_finish(ws.data_ptr(), out.data_ptr(), rows * N, _stream()), "b200_splitk_finish")
-    except Exception:
-        _splitk_ws.pop(_device_index(a.device), None)      # its contents are unknown now: start from a fresh one
-        _splitk_cnt.pop(_device_index(a.device), None)
-        raise
+    rc = lib.b200_gemm_skinny(a.data_ptr(), b.data_ptr(), out.data_ptr(), rows, N, K, splitk_factor(N, K), a.stride(0),
+                              b.stride(0), N, status_word(a.device).data_ptr(), _stream())
+    _check(rc, "b200_gemm_skinny")
     return out
-
-
-_splitk_ws: dict[int, torch.Tensor] = {}
-_splitk_cnt: dict[int, torch.Tensor] = {}
-
-
-def _splitk_counters(device: torch.device) -> torch.Tensor:
-    """One uint32 per output tile of a fused split-K product (N up to 2^20 columns); zero between launches."""
-
-    key = _device_index(device)
-    cnt = _splitk_cnt.get(key)
-    if cnt is None:
-        cnt = torch.zeros(8192, dtype=torch.int32, device=device)
-        _splitk_cnt[key] = cnt
-    return cnt
-
-
-def _device_index(device: torch.device) -> int:
-    return device.index if device.index is not None else torch.cuda.current_device()
-
-
-def _splitk_workspace(numel: int, device: torch.device) -> torch.Tensor:
-    key = _device_index(device)
-    ws = _splitk_ws.get(key)
-    if ws is None or ws.numel() < numel:
-        ws = torch.zeros(max(numel, 1 << 20), dtype=torch.float32, device=device)
-        _splitk_ws[key] = ws
-    return ws
 
 
 def _scale_is_bf16(*scales: torch.Tensor | None) -> int:

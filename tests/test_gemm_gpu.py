@@ -160,3 +160,28 @@ def test_gram_is_symmetric_and_exact(d, K, batch):
     assert (q.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
     with pytest.raises(native.KernelError):
         native.gram(x[:, :, :4] if d != 4 else x)
+
+
+# rows on both sides of each tile width, weight rows and K that are no multiple of a tile or of the slices, one slice to
+# eight, output widths that are no multiple of four
+@pytest.mark.parametrize("rows", [1, 16, 17, 33, 64, 100, 128])
+@pytest.mark.parametrize("n,k", [(8, 64), (130, 128), (2048, 2048), (1000, 1856), (11264, 512), (2046, 320), (333, 704)])
+def test_skinny_products(rows, n, k):
+    from research_b200.ops import native
+
+    torch.manual_seed(rows + n)
+    x = torch.randn(rows, k + 8, device="cuda").bfloat16()[:, :k]
+    w = (torch.randn(n, k, device="cuda") * 0.05).bfloat16()
+    y = native.gemm_skinny(x, w)
+    again = native.gemm_skinny(x, w)
+    native.check_status()
+    ref = x.double() @ w.double().t()
+    assert y.shape == (rows, n) and torch.equal(y, again)
+    assert (y.double() - ref).norm() <= 2.0 ** -8 * ref.norm()           # one rounding to bf16
+    lib = native.load()
+    for slices in (1, 2, 4, 8):                                          # more slices than blocks of K leave some empty
+        out = torch.full((rows, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+        assert lib.b200_gemm_skinny(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, n, k, slices, x.stride(0), k, n,
+                                    native.status_word(x.device).data_ptr(), native._stream()) == 0
+        assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+    native.check_status()
