@@ -24,6 +24,7 @@
 // of the identity on the way out, which makes a Newton-Schulz step three launches without an element-wise pass.
 // Eight matrices of 2048 x 2048: a Gram 106 -> 71 us, five steps 1823 -> 1248 us; of 5632 x 2048: 3566 -> 2644 us.
 #include "b200.cuh"
+#include "gemm_pair.cuh"
 #include "host_util.cuh"
 
 using namespace b200;
@@ -484,13 +485,31 @@ extern "C" int b200_gemm_bf16_grouped_k(const void* A, const void* B, void* C, i
                    accumulate, 0, nullptr, k_range, status, stream);
 }
 
+static int pair_tiles(int M, int N) {
+  return ((M + b200pair::PAIR_M - 1) / b200pair::PAIR_M) * ((N + b200pair::PAIR_N - 1) / b200pair::PAIR_N);
+}
+// CTA pairs pay where the product is long enough to run into the power limit and their coarser tiles leave no longer
+// last wave: 8192 x 11264 x 2048 330 -> 301 us, 2999 x 28672 x 4096 615 -> 556 us, 8192 x 2048 x 2048 60.8 -> 60.1 us;
+// 4096 x 3072 x 1024 (1.3e10 multiply-adds) 26.2 -> 26.5 us, 2048^3 (0.9e10) 17.1 -> 18.8 us.  `madds`: of all batches.
+static bool use_pair(int M, int N, int batch, double madds, int bn_hint, bool grouped_rows) {
+  if (grouped_rows) return false;                    // a row tile of 128 has its own B
+  if (bn_hint == 512) return true;
+  if (bn_hint == 128 || bn_hint == 256 || N <= 128 || madds < 2.5e10) return false;
+  const int sms = b200host::sm_count(), pairs = sms / 2;
+  const int single = ((M + BM - 1) / BM) * ((N + 255) / 256) * batch;
+  return (pair_tiles(M, N) * batch + pairs - 1) / pairs <= (single + sms - 1) / sms;
+}
+
 static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K, int batch, int batch_a, int batch_b,
                      int batch_c, long long lda, long long ldb, long long ldc, long long stride_a, long long stride_b,
                      long long stride_c, int a_mn, int b_mn, int out_f32, int accumulate, int bn_hint,
                      const int* tile_group, const int* k_range, int* status, void* stream, int c_shared, int k_total) {
   using namespace b200host;
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return RC_BAD_SHAPE;
-  const int BN = (bn_hint == 128 || bn_hint == 256) ? bn_hint : (N > 128 ? 256 : 128);
+  // bn_hint: 128 or 256 = that tile width, 512 = CTA pairs, else whichever suits
+  const double madds = (double)M * N * K * (k_range ? 1 : batch);   // with k_range, K is that of all groups together
+  const bool pair = use_pair(M, N, batch, madds, bn_hint, tile_group != nullptr);
+  const int BN = pair ? 128 : ((bn_hint == 128 || bn_hint == 256) ? bn_hint : (N > 128 ? 256 : 128));
   CUtensorMap tmA, tmB, tmC;
   int rc;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -513,6 +532,12 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
     rc = make_map_3d(&tmC, bf, C, N, M, batch_c, ldc * 2, stride_c * 2, 64, 32);
   if (rc) return rc;
 
+  if (pair) {
+    const b200pair::PairParams q{M, N, K, batch, accumulate, status, k_range, c_shared};
+    const int tiles = pair_tiles(M, N) * batch, pairs = sm_count() / 2;
+    return b200pair::dispatch(a_mn, b_mn, out_f32, tmA, tmB, tmC, q, tiles < pairs ? tiles : pairs,
+                              reinterpret_cast<cudaStream_t>(stream));
+  }
   GemmParams p{M, N, K, batch, accumulate, status, tile_group, k_range, c_shared};
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * batch;
   const int grid = tiles < sm_count() ? tiles : sm_count();

@@ -185,3 +185,27 @@ def test_skinny_products(rows, n, k):
                                     native.status_word(x.device).data_ptr(), native._stream()) == 0
         assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
     native.check_status()
+
+
+# the product on CTA pairs (bn=512) against 64 bits: edges of its 256 x 256 tile, a second CTA without rows or columns,
+# K shorter than a block and longer than the ring, more tiles than pairs, batches, accumulation
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (128, 256, 64), (129 * 8, 264, 72), (256, 136, 448), (520, 1000, 1000),
+                                   (2304, 2560, 128)])
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
+def test_products_on_cta_pairs(M, N, K, ta, tb):
+    from research_b200.ops import native
+
+    torch.manual_seed(M + K)
+    for batch in (1, 3):
+        a = torch.randn((batch, K, M) if ta else (batch, M, K), device="cuda").bfloat16()
+        b = torch.randn((batch, N, K) if tb else (batch, K, N), device="cuda").bfloat16()
+        ad, bd = a.double(), b.double()
+        ref = (ad.transpose(1, 2) if ta else ad) @ (bd.transpose(1, 2) if tb else bd)
+        size = (ad.abs().transpose(1, 2) if ta else ad.abs()) @ (bd.abs().transpose(1, 2) if tb else bd.abs())
+        y = native.gemm(a, b, trans_a=ta, trans_b=tb, bn=512)
+        assert (y.double() - ref).norm() <= 2.0 ** -8 * ref.norm()       # one rounding to bf16
+        acc = torch.full((batch, M, N), 0.5, device="cuda")
+        native.gemm(a, b, trans_a=ta, trans_b=tb, out=acc, accumulate=True, bn=512)
+        native.check_status()
+        # fp32 sums of K exact products: K * 2^-24 of the sum of magnitudes bounds any order
+        assert (acc.double() - ref - 0.5).abs().max() <= K * 2.0 ** -24 * (size.max() + 1)
