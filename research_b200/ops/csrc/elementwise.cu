@@ -217,24 +217,6 @@ rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
   }
 }
 
-// Tail of a split-K GEMM for a handful of rows: the slices were reduce-added into an fp32 workspace that was zero
-// before; this reads the sums, writes them as bf16 and puts the zeros back, so the workspace needs no separate
-// fill before its next use.  n % 4 == 0.
-__global__ void __launch_bounds__(256)
-splitk_finish_kernel(float* __restrict__ ws, __nv_bfloat16* __restrict__ out, long long n4) {
-  b200::pdl_launch_dependents();
-  b200::pdl_wait();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    const float4 v = reinterpret_cast<const float4*>(ws)[i];
-    reinterpret_cast<float4*>(ws)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    uint2 packed;
-    packed.x = *reinterpret_cast<uint32_t*>(&lo);
-    packed.y = *reinterpret_cast<uint32_t*>(&hi);
-    reinterpret_cast<uint2*>(out)[i] = packed;
-  }
-}
-
 // RMSNorm backward.  dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres if given); dw += sum_rows dy*xhat
 // Any H % 8 == 0: one warp per row, the dw partial sums of a block go through shared-memory atomics.
 template <typename W>
