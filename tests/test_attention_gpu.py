@@ -225,3 +225,23 @@ def test_attn_context_parallel_offsets(docs):
     native.check_status()
     assert (dk_sum - dk_full.float()).abs().max() <= 3e-2 * dk_full.float().abs().max() + 3e-2
     assert (dv_sum - dv_full.float()).abs().max() <= 3e-2 * dv_full.float().abs().max() + 3e-2
+
+
+# delta = sum over D of dO * O, seen through dQ: one head to more than a warp takes at once, tokens few enough that a token's
+# heads go to several warps and enough that they do not
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("B,S,H", [(1, 1, 1), (1, 130, 3), (2, 100, 20), (1, 70, 33), (3, 1700, 5), (1, 5000, 9)])
+def test_attn_bwd_head_counts(B, S, H, D):
+    from research_b200.ops import native
+
+    q, k, v, g = (_bf((B, S, H, D), i) for i in (1, 2, 3, 4))
+    o, lse = native.attn_fwd(q, k, v, causal=True)
+    dq, dk, dv = native.attn_bwd(q, k, v, o, g, lse, causal=True)
+    native.check_status()
+    leaves = [t.float().requires_grad_() for t in (q, k, v)]
+    ref = torch.nn.functional.scaled_dot_product_attention(*(t.transpose(1, 2) for t in leaves), is_causal=True)
+    ref.transpose(1, 2).backward(g.float())
+    for got, leaf in zip((dq, dk, dv), leaves):
+        # P, dS and the results are rounded to bf16 (2^-8 each) and O, which delta reads, before them: four roundings; at
+        # S == 1 the score gradients are zero and fp32 sums of D terms are left of them
+        assert (got.float() - leaf.grad).norm() <= 4 * 2.0 ** -8 * leaf.grad.norm() + 1e-4 * (H * D) ** 0.5 * (S == 1)
