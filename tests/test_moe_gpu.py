@@ -135,3 +135,35 @@ def test_native_routing_plan_matches_sort_based_dispatch(capacity):
     for name, u, v in zip(names, a, b):
         tol = 0.03 * v.abs().max().item() + 1e-3
         assert (u - v).abs().max().item() <= tol, (name, (u - v).abs().max().item(), tol)
+
+
+# widths around one and four 256-column steps of a lane's loads, choices around four rows at a time, with dropped choices
+@pytest.mark.parametrize("H", [8, 248, 264, 1016, 1032, 2056])
+@pytest.mark.parametrize("k,capacity", [(1, None), (3, 100), (4, None), (5, 64), (8, None)])
+def test_rows_to_experts_and_back(H, k, capacity):
+    from research_b200.ops import grouped, native
+
+    torch.manual_seed(H + k)
+    T, E = 200, 16
+    ids = torch.rand(T, E, device="cuda").topk(k, 1).indices
+    plan = grouped.RoutingPlan(ids, E, capacity)
+    x = torch.randn(T, H, device="cuda").bfloat16()
+    scale, w = torch.rand(T * k, device="cuda"), torch.rand(T * k, device="cuda")
+    src, dest = plan.src[:plan.rows_pad].long(), plan.dest.long()
+    for s in (None, scale):
+        rows = grouped._gather_rows(x, s, plan)
+        at = src.clamp(min=0)
+        ref = x[at // k].float() * (1.0 if s is None else s[at, None])
+        assert torch.equal(rows, torch.where((src >= 0)[:, None], ref, torch.zeros_like(ref)).bfloat16())
+    pad = torch.randn(plan.rows_pad, H, device="cuda").bfloat16()
+    kept = (dest >= 0)[:, None]
+    picked = torch.where(kept, pad[dest.clamp(min=0)].double(), torch.zeros(1, device="cuda", dtype=torch.float64))
+    ref = (picked * w[:, None].double()).view(T, k, H)
+    y = grouped._combine_rows(pad, w, plan)
+    # fp32 sums of k products, then one rounding to bf16 (2^-8)
+    assert ((y.double() - ref.sum(1)).abs() <= 2.0 ** -8 * ref.sum(1).abs() + k * 2.0 ** -23 * ref.abs().sum(1)).all()
+    dw = torch.full((T * k,), float("nan"), device="cuda")
+    native._check(grouped._moe_lib().b200_moe_combine_dw(grouped._one_ptr(pad), 1, x.data_ptr(), plan.dest.data_ptr(),
+                                                         dw.data_ptr(), T * k, H, k, 0, native._stream()), "dw")
+    prod = picked * x.double().repeat_interleave(k, 0)
+    assert ((dw.double() - prod.sum(1)).abs() <= H * 2.0 ** -24 * prod.abs().sum(1)).all()
