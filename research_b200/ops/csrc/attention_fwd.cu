@@ -308,7 +308,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
     float m_ref = -1.0e30f;
     float l_sum = 0.f;
-    bool ok = j_end > j_begin;
+    // rows that no kv row is visible to, a whole tile of them here: O = 0 and LSE = -inf, as for single such rows below
+    const bool empty = j_end <= j_begin;
+    bool ok = q0 + t * TILE_M < p.S;
     for (int j = j_begin; j < j_end && ok; ++j) {
       const int kv0 = (kv_begin + j) * BLOCK_N;
       if (!mbar_wait_warp(&s_full[t], (j - j_begin) & 1, ab, ERR_WAIT_S_READY)) { ok = false; break; }
@@ -415,15 +417,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[t]);
     }
-    if (ok) ok = mbar_wait_warp(&pv_done[t], 0, ab, ERR_WAIT_O_READY);
+    if (ok && !empty) ok = mbar_wait_warp(&pv_done[t], 0, ab, ERR_WAIT_O_READY);
+    // an empty tile of a CTA that streams blocks for the other one: its Q tile, where O is staged, has to have landed
+    if (ok && empty && n_blocks > 0) ok = mbar_wait_warp(q_full, 0, ab, ERR_WAIT_FULL);
     if (ok) {
       tc_fence_after();
       const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
         uint32_t r[32];
-        tmem_ld_32x32b_x32(tO + c * 32, r);
-        tmem_ld_wait();
+        if (!empty) {
+          tmem_ld_32x32b_x32(tO + c * 32, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = 0u;
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           uint4 v;

@@ -103,6 +103,45 @@ def test_attn_fwd_edges(D, S, kind):
     assert (lse.double() - ref_lse).abs().max() < 1e-4
 
 
+# rows from `seen` on see nothing: the rest of a tile, the second tile of a CTA, whole CTAs, everything
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("S,seen", [(256, 128), (256, 0), (300, 129), (300, 256), (640, 256), (900, 513), (130, 1)])
+def test_attn_rows_that_see_nothing(monkeypatch, D, causal, S, seen):
+    """O = 0 and LSE = -inf there, no gradient from there, whatever the outputs' memory held."""
+
+    from research_b200.ops import native
+
+    B, Hq, Hkv = 2, 3, 1
+    q, k, v, g = _bf((B, S, Hq, D), 11), _bf((B, S, Hkv, D), 12), _bf((B, S, Hkv, D), 13), _bf((B, S, Hq, D), 14)
+    lo = torch.zeros(B, S, dtype=torch.int32, device="cuda")
+    lo[:, seen:] = S
+    empty = torch.empty
+
+    def of_nans(*args, **kwargs):
+        t = empty(*args, **kwargs)
+        return t.fill_(float("nan")) if t.is_floating_point() else t
+
+    monkeypatch.setattr(torch, "empty", of_nans)
+    o, lse = native.attn_fwd(q, k, v, causal=causal, lo=lo)
+    grads = native.attn_bwd(q, k, v, o, g, lse, causal=causal, lo=lo)
+    monkeypatch.undo()
+    native.check_status()
+    assert not o[:, seen:].any() and (lse[:, :, seen:] == float("-inf")).all()
+    leaves = [t.double().requires_grad_(True) for t in (q, k, v)]
+    scores = torch.einsum("bqhd,bkd->bhqk", leaves[0][:, :seen], leaves[1][:, :, 0]) * D ** -0.5
+    if causal:
+        scores = scores.masked_fill(torch.ones(seen, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref_o = torch.einsum("bhqk,bkd->bqhd", scores.softmax(-1), leaves[2][:, :, 0])
+    ref = torch.autograd.grad([ref_o], leaves, [g[:, :seen].double()])
+    # P, dS, O and the results are rounded to bf16 (2^-8 each).  A causal row that sees one key has dS = 0 and what O's
+    # rounding leaves of dP - delta: 2^-9 |dO| |v| / sqrt(D) = 0.02, times |k| = 11 in two sequences of three heads at most
+    assert (o[:, :seen].double() - ref_o).norm() <= 2.0 ** -7 * ref_o.norm()
+    assert (lse[:, :, :seen].double() - scores.logsumexp(-1)).abs().le(1e-4).all()
+    for got, want in zip(grads, ref):
+        assert (got.double() - want).norm() <= 4 * 2.0 ** -8 * want.norm() + 0.7 * (seen == 1)
+
+
 @pytest.mark.parametrize("D", [128, 64])
 def test_attn_fwd_jumping_maxima_and_nonfinite(D):
     """Row maxima that jump by far more than the lazy rule tolerates, late and more than once; a NaN in one key reaches
