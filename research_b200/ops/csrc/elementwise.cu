@@ -469,8 +469,8 @@ __device__ __forceinline__ void qk_angles(const QkShape& q, const int* positions
 template <int LPH, typename W>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kQkFwdBlocks)
 qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride, __nv_bfloat16* __restrict__ out,
-                       long long out_stride, const W* __restrict__ w_first, const W* __restrict__ w_rest,
-                       const int* __restrict__ positions, float* __restrict__ rstd_out, const QkShape q, float eps) {
+                       long long out_stride, const W* w_first, const W* w_rest, const int* __restrict__ positions,
+                       float* __restrict__ rstd_out, const QkShape q, float eps) {
   constexpr int HPW = 32 / LPH, BATCH = 2;
   const int lane = threadIdx.x & 31;
   const int sub = lane / LPH, l = lane % LPH;
@@ -481,10 +481,9 @@ qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_stride
   float inv_freq[4], wv[8] = {1, 1, 1, 1, 1, 1, 1, 1};
 #pragma unroll
   for (int i = 0; i < 4; ++i) inv_freq[i] = exp2f(-q.log2_theta * (2.f * (float)(l * 4 + i)) / (float)q.D);
-  // the norm scales are weights (no predecessor writes them): they are read before the wait for the predecessor
-  if (norm && has_cols) load8w(w + l * 8, wv);
   b200::pdl_launch_dependents();   // no-ops unless launched as a dependent (decode steps)
   b200::pdl_wait();
+  if (norm && has_cols) load8w(w + l * 8, wv);   // no __restrict__: a load that may not move above the wait
   for (QkWalk<LPH> k(q, first); k.item < k.items; k.item += k.step) {
     int u0, u1;
     const long long t = k.at(q, u0, u1);

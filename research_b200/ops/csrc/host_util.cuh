@@ -75,7 +75,8 @@ inline int pdl_enabled() {
 
 // Launch with programmatic dependent launch when `pdl` is set: the kernel may become resident while its predecessor
 // in the stream is still running, and everything it reads or writes that the predecessor also touches must come
-// after its `griddepcontrol.wait` (b200.cuh: pdl_wait), which returns when the predecessor has completed.  A
+// after its `griddepcontrol.wait` (b200.cuh: pdl_wait), which returns when the predecessor has completed.  Weights and
+// norm scales count: what runs before is the caller's, and may be the cast or the copy that makes them.  A
 // predecessor lets this happen early by executing `griddepcontrol.launch_dependents` (pdl_launch_dependents) in
 // every CTA; without it the dependent launch begins when the predecessor's last CTA has exited.
 template <typename... KArgs, typename... Args>

@@ -3,8 +3,8 @@
 // tokens its columns (16, 32, 64 or 128, no padding to 128 rows), and K is cut over the CTAs of a cluster so that about
 // two CTAs per SM stream at once:
 //   warp 0     TMA producer: 128 x 64 tiles of W and the matching 64 columns of x through a ring
-//              of 3 to 12 stages; launched as a programmatic dependent, it requests its first W tiles before it waits for
-//              the predecessor, whose output only x depends on
+//              of 2 to 12 stages; launched as a programmatic dependent, it has its first W tiles brought into L2 before it
+//              waits for the predecessor, and reads W and x after that
 //   warp 1     MMA issuer: D[n][token] += W x^T in tensor memory
 //   warps 2-5  move the partial D to shared memory, token by token
 // The CTAs of a cluster then each sum 128 / cluster rows of D over all partials, read from one another's shared memory in
@@ -93,19 +93,15 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     if (elect_one()) {
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
-      auto load_w = [&](int i, int s) {
-        mbar_expect_tx(&full[s], STAGE_BYTES);
-        tma_load_2d(smem + s * STAGE_BYTES, &tmW, &full[s], (kb0 + i) * BK, tile * TILE_N);
-      };
-      const int ahead = min(n_kb, p.stages);
-      for (int i = 0; i < ahead; ++i) load_w(i, i);
+      // The predecessor may be what writes W (the cast of an fp32 parameter, a copy into it): W is read after the wait
+      // like x, and only brought into L2 ahead of it.
+      for (int i = 0; i < min(n_kb, p.stages); ++i) tma_prefetch_l2_2d(&tmW, (kb0 + i) * BK, tile * TILE_N);
       pdl_wait();
       bool ok = true;
       for (int i = 0, s = 0, ph = 1; i < n_kb; ++i) {
-        if (i >= ahead) {
-          if (!mbar_wait(&empty[s], ph, ab, ERR_WAIT_EMPTY)) { ok = false; break; }
-          load_w(i, s);
-        }
+        if (!mbar_wait(&empty[s], ph, ab, ERR_WAIT_EMPTY)) { ok = false; break; }
+        mbar_expect_tx(&full[s], STAGE_BYTES);
+        tma_load_2d(smem + s * STAGE_BYTES, &tmW, &full[s], (kb0 + i) * BK, tile * TILE_N);
         tma_load_2d(smem + s * STAGE_BYTES + W_BYTES, &tmX, &full[s], (kb0 + i) * BK, 0);
         if (++s == p.stages) {
           s = 0;

@@ -327,3 +327,26 @@ def test_fast_muon_section_matches_reference_path(family):
             continue
         # reference envelope for bf16 Newton-Schulz reorderings: update error <= 6e-4 at lr 1e-3 per step
         assert diff <= 2 * 6e-4 * (lr / 1e-3) + 1e-6, name
+
+
+def test_qknorm_scales_that_the_predecessor_writes():
+    """Scales straight out of a launch that lets its successor start early: bit for bit what they give with the device
+    idle in between."""
+
+    from research_b200.ops import native
+
+    x, raw = _bf((200, 8 * 128), 51), [_bf((2, 128), 52 + i, 1.0 + i) for i in range(4)]
+    ones, pos = torch.ones(128, device="cuda"), torch.arange(200, device="cuda", dtype=torch.int32)
+    runs = []
+    for idle in (True, False):
+        got = []
+        for i in range(32):
+            scales = native.rmsnorm_fwd(raw[i % 4], ones, 1e-6)[0]
+            if idle:
+                torch.cuda.synchronize()
+            out = torch.empty(200, 6 * 128, dtype=torch.bfloat16, device="cuda")
+            native.qknorm_rope_fwd_qk(x, out, scales[0], scales[1], pos, 4, 2, 128, 1e-6, 10000.0, True)
+            got.append(out)
+        runs.append(got)
+    native.check_status()
+    assert all(torch.equal(u, v) for u, v in zip(*runs))

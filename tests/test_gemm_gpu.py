@@ -187,6 +187,39 @@ def test_skinny_products(rows, n, k):
     native.check_status()
 
 
+@pytest.mark.parametrize("rows,n,k", [(1, 128, 2048), (32, 2048, 4096), (64, 512, 512)])
+def test_skinny_product_with_weights_that_its_predecessor_writes(rows, n, k):
+    """W straight out of another such product, and an fp32 parameter that is cast on every call: bit for bit what it
+    is with the device idle before each product."""
+
+    from research_b200.ops import functional as Fn
+    from research_b200.ops import native
+
+    torch.manual_seed(k)
+    x = torch.randn(rows, k, device="cuda").bfloat16()
+    a = torch.randn(128, 512, device="cuda").bfloat16()
+    b = [(torch.randn(k, 512, device="cuda") * 0.05).bfloat16() for _ in range(4)]
+    start = torch.randn(n, k, device="cuda") * 0.05
+    p = torch.nn.Parameter(start.clone())
+    runs = []
+    with torch.no_grad():
+        for idle in (True, False):
+            p.copy_(start)
+            got = []
+            for i in range(24):
+                w = native.gemm_skinny(a, b[i % 4])
+                if idle:
+                    torch.cuda.synchronize()
+                got.append(native.gemm_skinny(x, w))
+                p.mul_(-1.25 if i % 2 else 0.8)
+                if idle:
+                    torch.cuda.synchronize()
+                got.append(Fn.linear(x, p))
+            runs.append(got)
+    native.check_status()
+    assert all(torch.equal(u, v) for u, v in zip(*runs))
+
+
 # the product on CTA pairs (bn=512) against 64 bits: edges of its 256 x 256 tile, a second CTA without rows or columns,
 # K shorter than a block and longer than the ring, more tiles than pairs, batches, accumulation
 @pytest.mark.parametrize("M,N,K", [(8, 8, 8), (128, 256, 64), (129 * 8, 264, 72), (256, 136, 448), (520, 1000, 1000),

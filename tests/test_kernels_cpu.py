@@ -1,6 +1,7 @@
 """Kernel build cache and kernel plan, with the compiler replaced by a recorder and the tree by a temporary copy."""
 
 import json
+import re
 from pathlib import Path
 
 import pytest
@@ -179,3 +180,35 @@ def test_roofline_denominators_come_from_the_measured_file_or_the_stated_fallbac
     assert microbench.peaks() == {"hbm_gbs": 6500.0, "bf16_tflops": 1600.0, "source": "measured"}
     (tmp_path / "MEASURED_PEAKS.json").unlink()
     assert microbench.peaks() == {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "source": "fallback"}
+
+
+def _kernels_that_wait():
+    """(name, body) of every kernel that waits for its predecessor in the stream (programmatic dependent launch)."""
+
+    for path in sorted((build.PKG_ROOT / "ops" / "csrc").glob("*.cu*")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for head in re.finditer(r"__global__[^{]*?(\w+_kernel)\s*\([^{]*\{", text):
+            depth, at = 1, head.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[at], 0)
+                at += 1
+            if "pdl_wait()" in text[head.end():at]:
+                yield head.group(1), text[head.end():at]
+
+
+def test_dependent_kernels_read_nothing_before_their_wait():
+    """A kernel that starts before its predecessor has ended may read global memory only after its wait: the predecessor
+    can be what writes its weights or scales (a cast, a copy, a product) as well as its input."""
+
+    seen = []
+    for name, body in _kernels_that_wait():
+        seen.append(name)
+        if name == "attn_bwd_kernel":
+            # dK/dV beside dQ: all that it reads was complete before the dQ kernel, an ordinary launch, began; it waits
+            # only before it ends
+            assert body.rstrip("} \n").endswith("pdl_wait();")
+            continue
+        before = body[:body.index("pdl_wait()")]
+        reads = re.findall(r"tma_load_\w+|bulk_g2s|load8\w*|__ldg|\*reinterpret_cast<const", before)
+        assert not reads, (name, reads)
+    assert {"skinny_gemm_kernel", "qknorm_rope_fwd_kernel", "rmsnorm_fwd_row_kernel", "attn_bwd_kernel"} <= set(seen), seen
