@@ -80,7 +80,9 @@ class PagedKVCache:
         idx = positions.long()
         from_zero = T > 1 and (self._from_zero or bool(
             (positions == torch.arange(T, device=q.device, dtype=positions.dtype)).all()))
-        if from_zero and native_ok and kp.dtype == torch.bfloat16:
+        # one prompt for every sequence of the cache takes the block copies, which repeat its rows
+        same_rows = (B, *k.shape[2:]) == (kp.shape[0], kp.shape[2], kp.shape[4])
+        if from_zero and native_ok and same_rows and kp.dtype == torch.bfloat16:
             # prefill from position 0: the rows go to their pages in one launch and the flash kernel takes them where
             # they are (column ranges of the packed projection)
             from research_b200.ops import native

@@ -137,13 +137,17 @@ def kv_write_prompt_paged(k: torch.Tensor, v: torch.Tensor, k_pool: torch.Tensor
     """Write rows ``0 .. T-1`` of every sequence (``k`` / ``v``: ``[B, T, Hkv, D]`` views with dense heads) into
     head-major paged caches ``[B, pages, Hkv, page_rows, D]``."""
 
-    lib = native.load()
     B, T, Hkv, D = k.shape
     for t in (k, v):
         if t.dtype != torch.bfloat16 or t.stride(3) != 1 or t.stride(2) != D:
             raise KernelError("k / v must be bf16 [B,T,Hkv,D] views with heads D elements apart")
-    if v.shape != k.shape or T > k_pool.shape[1] * k_pool.shape[3] or not (k_pool.is_contiguous() and v_pool.is_contiguous()):
-        raise KernelError("the prompt does not fit the paged caches, or they are not contiguous")
+    for pool in (k_pool, v_pool):
+        if pool.dtype != torch.bfloat16 or not pool.is_contiguous() or (
+                (pool.shape[0], pool.shape[2], pool.shape[4]) != (B, Hkv, D) or T > pool.shape[1] * pool.shape[3]):
+            raise KernelError(f"a prompt {tuple(k.shape)} does not fit contiguous bf16 paged caches {tuple(pool.shape)}")
+    if v.shape != k.shape or v_pool.shape != k_pool.shape:
+        raise KernelError("k and v, and their caches, must have one shape")
+    lib = native.load()
     rc = lib.b200_kv_write_prompt(k.data_ptr(), v.data_ptr(), k.stride(1), k.stride(0) if B > 1 else 0, v.stride(1),
                                   v.stride(0) if B > 1 else 0, k_pool.data_ptr(), v_pool.data_ptr(), k_pool.stride(0),
                                   k_pool.stride(2), k_pool.stride(1), k_pool.shape[3], B, T, Hkv, D, native._stream())

@@ -220,6 +220,31 @@ def test_prompt_rows_in_pages(T, B, Hkv, D):
     assert not told._from_zero
 
 
+# lengths around a page: fewer rows than one, a whole one, one row more
+@pytest.mark.parametrize("T", [2, 128, 129])
+def test_one_prompt_for_every_sequence_of_a_cache(T):
+    """A single prompt written into a cache of several sequences goes to all of them, as in the block copies; any
+    other number of prompts that is not the cache's is refused."""
+
+    from research_b200.infer.generation import PagedKVCache
+    from research_b200.ops import native
+
+    make = lambda: PagedKVCache(layers=2, batch=3, max_len=T + 5, kv_heads=2, head_dim=64, page_size=128,  # noqa: E731
+                                dtype=torch.bfloat16, device=torch.device("cuda"))
+    q, k, v = (torch.randn(1, T, h, 64, device="cuda").bfloat16() for h in (4, 2, 2))
+    pos = torch.arange(T, device="cuda", dtype=torch.int32).expand(1, T).contiguous()
+    cache = make()
+    with cache.prompt():
+        o = cache.update_and_attend(1, q, k, v, pos, None)
+    native.check_status()
+    assert torch.equal(o, native.attn_fwd(q, k, v)[0].reshape(1, T, -1))
+    assert torch.equal(cache._rows(cache.k, 1, T), k.expand(3, T, 2, 64)) and not cache.k[0].any()
+    assert torch.equal(cache._rows(cache.v, 1, T), v.expand(3, T, 2, 64))
+    for n in (2, 4):
+        with pytest.raises(RuntimeError):
+            make().update_and_attend(0, *(t.expand(n, *t.shape[1:]) for t in (q, k, v)), pos.expand(n, T).contiguous(), None)
+
+
 @pytest.mark.parametrize("S,n,off", [(1, 1, 0), (5, 3, 0), (129, 300, 128), (1000, 1000, 0)])
 def test_kv_upper_bound_matches_a_search(S, n, off):
     from research_b200.ops import native

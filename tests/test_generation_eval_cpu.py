@@ -56,6 +56,19 @@ def test_cache_prefill_block_copy_equals_scatter_write(prompt):
     assert torch.equal(blocked._rows(blocked.k, 0, prompt), k)
 
 
+@pytest.mark.parametrize("shape", [(2, 5, 2, 64), (1, 5, 2, 64), (4, 5, 2, 64), (3, 5, 1, 64), (3, 5, 2, 128), (3, 9, 2, 64)])
+def test_prompt_rows_that_do_not_match_the_cache_are_refused_before_any_launch(shape):
+    """3 sequences of two pages of 4 rows, 2 heads of 64."""
+
+    from research_b200.errors import KernelError
+    from research_b200.ops.decode import kv_write_prompt_paged
+
+    rows = torch.zeros(shape, dtype=torch.bfloat16)
+    pool = torch.zeros(3, 2, 2, 4, 64, dtype=torch.bfloat16)
+    with pytest.raises(KernelError, match="does not fit"):
+        kv_write_prompt_paged(rows, rows, pool, pool.clone())
+
+
 def test_cache_window_limits_the_keys_a_query_sees():
     torch.manual_seed(0)
     B, T, H, D = 1, 8, 1, 4
