@@ -10,7 +10,7 @@ components/attention.py:213-218).
 
 from __future__ import annotations
 
-from contextlib import contextmanager
+from contextlib import contextmanager, nullcontext
 from dataclasses import dataclass
 
 import torch
@@ -21,6 +21,8 @@ from research_b200.ops import functional as Fn
 
 class PagedKVCache:
     """``[layers, pages, kv_heads, page_size, head_dim]`` K and V pools (head-major pages) + a page table."""
+
+    _from_zero = False
 
     def __init__(self, *, layers: int, batch: int, max_len: int, kv_heads: int, head_dim: int, page_size: int,
                  dtype: torch.dtype, device: torch.device):
@@ -34,7 +36,6 @@ class PagedKVCache:
         self.page_table = torch.arange(total_pages, device=device, dtype=torch.int32).view(batch, self.pages_per_seq)
         self.lengths = torch.zeros(batch, dtype=torch.int32, device=device)
         self.batch = batch
-        self._from_zero = False
 
     @contextmanager
     def prompt(self):
@@ -233,7 +234,8 @@ def prefill(model, prompt_ids: torch.Tensor, cache: PagedKVCache) -> torch.Tenso
     B, P = prompt_ids.shape
     device = next(model.parameters()).device
     positions = torch.arange(P, device=device, dtype=torch.int32).expand(B, P).contiguous()
-    with cache.prompt():
+    # any object that stores rows and attends over them will do
+    with cache.prompt() if isinstance(cache, PagedKVCache) else nullcontext():
         logits = model.run_with_cache(prompt_ids.to(device=device, dtype=torch.int32), positions, cache, last_only=True)
     cache.advance(positions)
     return logits[:, -1]

@@ -9,7 +9,7 @@ import torch
 from research_b200.config import run_spec_from_mapping
 from research_b200.config.specs import MoeBalanceSpec, ScheduleSpec
 from research_b200.errors import ContractError
-from research_b200.infer.generation import PagedKVCache, generate_tokens, init_kv_cache, sample_next_token
+from research_b200.infer.generation import PagedKVCache, generate_tokens, init_kv_cache, prefill, sample_next_token
 from research_b200.models.build import build_model
 from research_b200.optim.schedules import build_lr_schedule
 from research_b200.steps.eval import causal_lm_loss
@@ -67,6 +67,20 @@ def test_prompt_rows_that_do_not_match_the_cache_are_refused_before_any_launch(s
     pool = torch.zeros(3, 2, 2, 4, 64, dtype=torch.bfloat16)
     with pytest.raises(KernelError, match="does not fit"):
         kv_write_prompt_paged(rows, rows, pool, pool.clone())
+
+
+def test_prefill_takes_any_cache_that_stores_and_attends():
+    """A program's own cache needs ``update_and_attend`` and ``advance``, no more."""
+
+    model = _model()[0].model.eval()
+    prompt = torch.randint(0, model.spec.vocab_size, (2, 5))
+    paged = init_kv_cache(model, 2, 8, page_size=4)
+
+    class Mine:
+        update_and_attend, advance = paged.update_and_attend, paged.advance
+
+    assert torch.equal(prefill(model, prompt, Mine()), prefill(model, prompt, init_kv_cache(model, 2, 8, page_size=4)))
+    assert paged.lengths.tolist() == [5, 5]
 
 
 def test_cache_window_limits_the_keys_a_query_sees():
