@@ -400,8 +400,7 @@ int dispatch(bool a_mn, bool b_mn, bool out_f32, const CUtensorMap& tmA, const C
 static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K, int batch, int batch_a, int batch_b,
                      int batch_c, long long lda, long long ldb, long long ldc, long long stride_a, long long stride_b,
                      long long stride_c, int a_mn, int b_mn, int out_f32, int accumulate, int bn_hint,
-                     const int* tile_group, const int* k_range, int* status, void* stream, int c_shared = 0,
-                     int k_total = 0);
+                     const int* tile_group, const int* k_range, int* status, void* stream, int c_shared = 0);
 
 extern "C" int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int batch, long long lda,
                               long long ldb, long long ldc, long long stride_a, long long stride_b,
@@ -412,17 +411,14 @@ extern "C" int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int 
 }
 
 // Split-K for any operand layout with an fp32 output that is accumulated into (weight gradients: the contraction
-// runs over tokens and is long, the output has few tiles, and the partial sums are reduce-added anyway).  Slices are
-// whole 64-element blocks of K; the last may be shorter.
+// runs over tokens and is long, the output has few tiles, and the partial sums are reduce-added anyway).  The slices
+// are equal and whole 64-element blocks of K.
 extern "C" int b200_gemm_bf16_splitk_acc(const void* A, const void* B, void* C, int M, int N, int K, int splits,
                                          long long lda, long long ldb, long long ldc, int a_mn, int b_mn, int* status,
                                          void* stream) {
-  if (splits < 1 || K < 1) return b200host::RC_BAD_SHAPE;
-  const int blocks = (K + BK - 1) / BK;
-  const int per = (blocks + splits - 1) / splits;
-  splits = (blocks + per - 1) / per;   // no slice is empty
-  return gemm_impl(A, B, C, M, N, per * BK, splits, 1, 1, 1, lda, ldb, ldc, 0, 0, 0, a_mn, b_mn, 1, 1, 0, nullptr,
-                   nullptr, status, stream, 1, K);
+  if (splits < 1 || K % (BK * splits)) return b200host::RC_BAD_SHAPE;
+  return gemm_impl(A, B, C, M, N, K / splits, splits, 1, 1, 1, lda, ldb, ldc, 0, 0, 0, a_mn, b_mn, 1, 1, 0, nullptr,
+                   nullptr, status, stream, 1);
 }
 
 // C[b] = alpha * A[b] A[b]^T + beta * G[b] + gamma * I for a stack of matrices, each C[b] a symmetric d x d matrix of
@@ -503,7 +499,7 @@ static bool use_pair(int M, int N, int batch, double madds, int bn_hint, bool gr
 static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K, int batch, int batch_a, int batch_b,
                      int batch_c, long long lda, long long ldb, long long ldc, long long stride_a, long long stride_b,
                      long long stride_c, int a_mn, int b_mn, int out_f32, int accumulate, int bn_hint,
-                     const int* tile_group, const int* k_range, int* status, void* stream, int c_shared, int k_total) {
+                     const int* tile_group, const int* k_range, int* status, void* stream, int c_shared) {
   using namespace b200host;
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return RC_BAD_SHAPE;
   // bn_hint: 128 or 256 = that tile width, 512 = CTA pairs, else whichever suits
@@ -513,8 +509,7 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
   CUtensorMap tmA, tmB, tmC;
   int rc;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  // split-K addresses slices through the K coordinate; what lies past the end of K reads as zero
-  const int k_map = k_total ? k_total : (c_shared ? K * batch : K);
+  const int k_map = c_shared ? K * batch : K;  // split-K addresses slices through the K coordinate
   if (c_shared) batch_a = batch_b = batch_c = 1;
   if (!a_mn)
     rc = make_map_3d(&tmA, bf, A, k_map, M, batch_a, lda * 2, stride_a * 2, BK, BM);

@@ -304,21 +304,21 @@ def gram(x: torch.Tensor, *, transposed: bool = False, alpha: float = 1.0, beta:
 # normalisation / activation / embedding / loss / optimizer
 # --------------------------------------------------------------------------------------------------
 @functools.lru_cache(maxsize=4096)
-def wave_splits(m: int, n: int, k: int, sms: int = 148, max_splits: int = 8, min_slice: int = 1024) -> int:
+def wave_splits(m: int, n: int, k: int, sms: int = 148, max_splits: int = 8) -> int:
     """K slices for an accumulated product: the count of least ``waves * (k blocks per slice * 0.4 + 3)``, that is
     microseconds at 0.4 per 64-element block of K of a 128 x 256 tile and 3 for what adding the fp32 tile to memory
     leaves uncovered.  Fewer slices win ties (3 %).  Measured with 8192 tokens: 11264 x 2048 1 / 2 / 4 / 8 slices 296 /
-    308 / 351 / 490 us, 2048 x 5632 206 / 182 / 201 / 239 us, 2048 x 2048 57 / 59 / 64 / 67 us; with 1024 tokens
-    2048 x 512 13.8 / 11.0 / 9.5 / 12.8 us.  Slices are at least ``min_slice`` long; from 1024 on they divide ``k``."""
+    308 / 351 / 490 us, 2048 x 5632 206 / 182 / 201 / 239 us, 2048 x 2048 57 / 59 / 64 / 67 us.  The slices divide ``k``
+    into whole blocks and are at least 1024 long, and a single tile is not cut in two: everything else stays one pass,
+    whose sums are the same bits every time (1024 tokens, 2048 x 512: 13.8 us, 9.5 with four slices)."""
 
     tiles = ((m + 127) // 128) * ((n + 255) // 256)
     kblocks = (k + 63) // 64
     best, best_cost = 1, float("inf")
     for s in range(1, max_splits + 1):
-        per = -(-kblocks // s)
-        if s > 1 and (per * 64 < min_slice or -(-kblocks // per) != s or (min_slice >= 1024 and kblocks % s)):
+        if s > 1 and (k % (64 * s) or k // s < 1024 or tiles * s < 3):
             continue
-        cost = -(-tiles * s // sms) * (per * 0.4 + 3.0)
+        cost = -(-tiles * s // sms) * (kblocks // s * 0.4 + 3.0)
         if cost < 0.97 * best_cost:
             best, best_cost = s, cost
     return best
@@ -326,15 +326,16 @@ def wave_splits(m: int, n: int, k: int, sms: int = 148, max_splits: int = 8, min
 
 def gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, grad: torch.Tensor) -> None:
     """``grad[M, N] (fp32) += dy[K, M]^T @ x[K, N]`` with the contraction over tokens cut into slices where the output
-    has few tiles for the device (the partial sums are reduce-added into ``grad`` either way)."""
+    has few tiles for the device.  Slices are reduce-added into ``grad`` in arrival order; there are none with fewer
+    than 2048 tokens, a token count that is no multiple of 64, or in the deterministic mode."""
 
     K, M = dy.shape
     N = x.shape[1]
     splits = 1
     if (dy.stride(1) == 1 and x.stride(1) == 1 and grad.dim() == 2 and grad.stride(1) == 1
             and grad.dtype == torch.float32 and dy.dtype == x.dtype == torch.bfloat16 and x.shape[0] == K
-            and tuple(grad.shape) == (M, N) and not _DETERMINISTIC):         # slices are reduce-added in arrival order
-        splits = wave_splits(M, N, K, min_slice=128)
+            and tuple(grad.shape) == (M, N) and not _DETERMINISTIC):
+        splits = wave_splits(M, N, K)
     if splits == 1:
         gemm(dy, x, trans_a=True, trans_b=False, out=grad, accumulate=True)
         return

@@ -81,9 +81,27 @@ def test_dion2_kernel_size_rules():
 
 
 def test_wave_splits_fills_whole_waves_and_respects_the_slice_floor():
-    # 16 x 8 output tiles on 148 SMs: 128 tiles leave 20 SMs idle, a second K slice would need two waves for 256
-    assert native.wave_splits(2048, 2048, 32768) in (1, 2, 3, 4, 5, 6, 7, 8)
     assert native.wave_splits(128, 256, 1024) == 1                               # slices of at least 1024 rows
-    for m, n, k in [(2048, 2048, 32768), (4096, 2048, 32768), (2048, 8192, 16384)]:
-        s = native.wave_splits(m, n, k)
-        assert (k // 64) % s == 0 and k // s >= 1024
+    # 2048 x 5632 has 352 tiles: 2.4 waves of 148 in one slice, 4.8 of half the length in two; 2048 x 2048 has 128 and
+    # 11264 x 2048 704, whose last waves are nearly full
+    assert [native.wave_splits(m, n, 8192) for m, n in [(2048, 2048), (2048, 5632), (11264, 2048)]] == [1, 2, 1]
+    assert native.wave_splits(512, 256, 8192) == 8 and native.wave_splits(512, 256, 4096) == 4
+    for m in range(128, 6000, 640):
+        for n in range(256, 6000, 512):
+            for k in (64, 1000, 1024, 1984, 2047, 2048, 2999, 3072, 4096, 8200, 8256, 65536):
+                s = native.wave_splits(m, n, k)
+                assert s == 1 or (k % (64 * s) == 0 and k // s >= 1024), (m, n, k, s)
+
+
+def test_weight_gradients_are_one_pass_where_the_sums_have_to_repeat_themselves(monkeypatch):
+    """Fewer than 2048 tokens and token counts that are no multiple of 64 are never cut into slices, which are added in
+    arrival order."""
+
+    passes = []
+    monkeypatch.setattr(native, "gemm", lambda dy, x, **kw: passes.append(dy.shape[0]))
+    tokens = [1, 63, 64, 777, 1000, 1024, 1984, 2999, 4100]
+    for k in tokens:
+        for m, n in ((128, 256), (512, 512), (2048, 512)):
+            native.gemm_wgrad(torch.zeros(k, m, dtype=torch.bfloat16), torch.zeros(k, n, dtype=torch.bfloat16),
+                              torch.zeros(m, n))
+    assert passes == [k for k in tokens for _ in range(3)]
