@@ -281,20 +281,22 @@ def _matrix(t: torch.Tensor) -> tuple[int, int, int, int, int, int]:
 
 def gram(x: torch.Tensor, *, transposed: bool = False, alpha: float = 1.0, beta: float = 0.0,
          gamma: float = 0.0) -> torch.Tensor:
-    """``alpha * x x^T + beta * x + gamma * I`` (``transposed``: of ``x^T x``) for a contiguous bf16 stack ``[batch, m, n]``
-    with m and n multiples of 8; the result is symmetric bit for bit and half of it is computed.  ``beta`` needs a
-    stack of symmetric matrices."""
+    """``alpha * x x^T + beta * x + gamma * I`` (``transposed``: of ``x^T x``) for a bf16 matrix or stack ``[batch, m, n]``
+    with dense rows (m may be odd where the product is ``x^T x``, n and the size of the result are multiples of 8); the
+    result is symmetric bit for bit and half of it is computed.  ``beta`` needs contiguous symmetric matrices."""
 
     lib = load()
-    if x.dtype != torch.bfloat16 or x.dim() != 3 or not x.is_contiguous() or x.shape[1] % 8 or x.shape[2] % 8:
-        raise KernelError(f"gram needs a contiguous bf16 [batch, m, n] stack with m, n % 8 == 0, got {tuple(x.shape)}")
-    batch, m, n = x.shape
+    if x.dtype != torch.bfloat16 or x.dim() not in (2, 3):
+        raise KernelError(f"gram needs a bf16 matrix or stack of matrices, got {tuple(x.shape)} {x.dtype}")
+    batch, m, n, batch_stride, ld, dense = _matrix(x)
     d, K = (n, m) if transposed else (m, n)
-    if beta != 0.0 and m != n:
-        raise KernelError("gram: beta adds the input itself, which has to be square")
-    out = torch.empty((batch, d, d), dtype=x.dtype, device=x.device)
-    rc = lib.b200_gemm_bf16_sym(x.data_ptr(), x.data_ptr() if beta != 0.0 else None, out.data_ptr(), d, K, batch, n, d,
-                                m * n, d * d, int(transposed), alpha, beta, gamma,
+    if dense != 1 or d % 8 or n % 8 or (batch > 1 and batch_stride == 0):
+        raise KernelError(f"gram needs dense rows and sizes that are multiples of 8, got {tuple(x.shape)} {x.stride()}")
+    if beta != 0.0 and (m != n or not x.is_contiguous()):
+        raise KernelError("gram: beta adds the input itself, which has to be square and contiguous")
+    out = torch.empty((*x.shape[:-2], d, d), dtype=x.dtype, device=x.device)
+    rc = lib.b200_gemm_bf16_sym(x.data_ptr(), x.data_ptr() if beta != 0.0 else None, out.data_ptr(), d, K, batch, ld, d,
+                                batch_stride if batch > 1 else m * ld, d * d, int(transposed), alpha, beta, gamma,
                                 status_word(x.device).data_ptr(), _stream())
     _check(rc, "b200_gemm_bf16_sym")
     return out

@@ -165,6 +165,32 @@ def test_gram_is_symmetric_and_exact(d, K, batch):
         native.gram(x[:, :, :4] if d != 4 else x)
 
 
+# every form of stack that plain products take: rows that are no multiple of 8 where there are more rows than columns,
+# rows and matrices at a distance, a single matrix
+@pytest.mark.parametrize("shape", [(2, 1001, 512), (3, 130, 64), (2, 256, 520), (1, 70, 64), (300, 136), (136, 264)])
+@pytest.mark.parametrize("apart", [0, 8])
+def test_newton_schulz_takes_every_stack_that_products_take(shape, apart):
+    from research_b200.ops import native
+    from research_b200.optim import orthogonalize as orth
+
+    torch.manual_seed(shape[-1])
+    x = torch.randn(shape, device="cuda")
+    wide = torch.zeros(*shape[:-2], shape[-2] + apart, shape[-1] + apart, device="cuda", dtype=torch.bfloat16)
+    stack = wide[..., :shape[-2], :shape[-1]].copy_(x / torch.linalg.matrix_norm(x, keepdim=True))
+    got = orth.newton_schulz_stack_(stack)
+    native.check_status()
+    ref = stack.double()
+    if shape[-2] > shape[-1]:
+        ref = ref.transpose(-1, -2)
+    for _ in range(orth.MUON_NS_STEPS):
+        a, b, c = orth.MUON_NS_COEFFICIENTS
+        g = ref @ ref.transpose(-1, -2)
+        ref = a * ref + (b * g + c * g @ g) @ ref
+    ref = ref.transpose(-1, -2) if shape[-2] > shape[-1] else ref
+    # five steps, each with three roundings to bf16 that the next step's slope (up to 3.4445) amplifies
+    assert got.shape == stack.shape and (got.double() - ref).norm() <= 5 * 3 * 2.0 ** -8 * ref.norm()
+
+
 # rows on both sides of each tile width, weight rows and K that are no multiple of a tile or of the slices, one slice to
 # eight, output widths that are no multiple of four
 @pytest.mark.parametrize("rows", [1, 16, 17, 33, 64, 100, 128])
