@@ -380,7 +380,16 @@ rmsnorm_bwd_cols_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict
       reinterpret_cast<float4*>(dw_smem)[(t + v * threads) * 2 + i] =
           make_float4(acc[v][4 * i], acc[v][4 * i + 1], acc[v][4 * i + 2], acc[v][4 * i + 3]);
   __syncthreads();
-  for (int i = t; i < (H >> 2); i += threads) red_add4(dw + 4 * i, reinterpret_cast<const float4*>(dw_smem)[i]);
+  // dw may start anywhere in an arena: the elements up to the next 16 bytes and the last of the row by themselves
+  const int head = (4 - static_cast<int>((reinterpret_cast<uintptr_t>(dw) >> 2) & 3)) & 3;
+  for (int j = head + 4 * t; j + 4 <= H; j += 4 * threads) {
+    const float* v = dw_smem + j;
+    red_add4(dw + j, head ? make_float4(v[0], v[1], v[2], v[3]) : *reinterpret_cast<const float4*>(v));
+  }
+  if (head && t < 4) {
+    const int i = t < head ? t : H - 4 + t;
+    atomicAdd(dw + i, dw_smem[i]);
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1141,7 +1150,6 @@ extern "C" int b200_rmsnorm_fwd(const void* x, const void* delta, const void* w,
 template <typename W>
 static int rmsnorm_bwd_launch(const void* x, const W* w, const void* rstd, const void* dy, const void* dres, void* dx,
                               void* dw, int rows, int H, void* stream) {
-  const bool dw16 = (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
 #define RMS_BWD_COLS(VEC, ROWS, THREADS, MAXT, MINB, AHEAD)                                                           \
   do {                                                                                                                \
     rmsnorm_bwd_cols_kernel<VEC, ROWS, MAXT, MINB, AHEAD, W>                                                          \
@@ -1152,10 +1160,10 @@ static int rmsnorm_bwd_launch(const void* x, const W* w, const void* rstd, const
     return LAST_ERR();                                                                                                \
   } while (0)
   // whole warps of columns: one 16-byte vector of a row per thread up to 2048 columns, two above
-  if (dw16 && H % 256 == 0 && H <= 512) RMS_BWD_COLS(1, 4, H / 8, 64, 8, false);
-  if (dw16 && H % 256 == 0 && H <= 2048) RMS_BWD_COLS(1, 2, H / 8, 256, 4, false);
-  if (dw16 && H % 512 == 0 && H <= 4096) RMS_BWD_COLS(2, 1, H / 16, 256, 3, false);
-  if (dw16 && H % 512 == 0 && H <= 8192) RMS_BWD_COLS(2, 1, H / 16, 512, 1, true);
+  if (H % 256 == 0 && H <= 512) RMS_BWD_COLS(1, 4, H / 8, 64, 8, false);
+  if (H % 256 == 0 && H <= 2048) RMS_BWD_COLS(1, 2, H / 8, 256, 4, false);
+  if (H % 512 == 0 && H <= 4096) RMS_BWD_COLS(2, 1, H / 16, 256, 3, false);
+  if (H % 512 == 0 && H <= 8192) RMS_BWD_COLS(2, 1, H / 16, 512, 1, true);
 #undef RMS_BWD_COLS
   const int grid = grid_for((long long)rows, kWarpsPerBlock, 2);
   rmsnorm_bwd_kernel<W><<<grid, kWarpsPerBlock * 32, H * sizeof(float), STREAM(stream)>>>(

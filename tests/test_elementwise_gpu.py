@@ -87,6 +87,42 @@ def test_rmsnorm_bwd_widths(H, rows, with_res):
     assert _off(dw, wr.grad + 1) < 1e-5
 
 
+# a weight gradient that starts anywhere in an arena: the same values, by the same kernel
+@pytest.mark.parametrize("H", [256, 512, 1024, 2048, 4096, 8192])
+def test_rmsnorm_bwd_into_an_unaligned_gradient(H):
+    from research_b200.ops import native
+
+    rows = 2 ** 25 // H
+    x, dy, w = _bf((rows, H), 31), _bf((rows, H), 32), torch.rand(H, device="cuda") + 0.5
+    _, rstd, _ = native.rmsnorm_fwd(x, w, 1e-6)
+    arena = torch.zeros(H + 8, device="cuda")
+
+    def run(off):
+        return native.rmsnorm_bwd(x, w, rstd, dy, arena[off:off + H])
+
+    def time_us(off):
+        best = float("inf")
+        for _ in range(5):
+            s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            s.record()
+            for _ in range(10):
+                run(off)
+            e.record()
+            torch.cuda.synchronize()
+            best = min(best, s.elapsed_time(e) * 100)
+        return best
+
+    want_dx, want = run(0), arena[:H].clone()
+    for off in (1, 2, 3):
+        arena.zero_()
+        assert torch.equal(run(off), want_dx)
+        # fp32 partial sums of at most 2368 blocks in arrival order
+        assert _off(arena[off:off + H], want) < 1e-4 and not arena[:off].any() and not arena[off + H:].any()
+    # the kernel that walks rows with a warp each takes 1.3 (256 columns) to 3.3 times as long
+    slow, fast = time_us(1), time_us(0)
+    assert slow < 1.2 * fast, (slow, fast)
+
+
 # odd head counts, tokens on both sides of the rule that deals a token's heads to several warps (4736 tokens)
 @pytest.mark.parametrize("T,hq,hkv,D", [(1, 1, 1, 128), (33, 3, 1, 64), (700, 5, 3, 128), (700, 7, 1, 96),
                                         (4735, 2, 1, 64), (4740, 3, 2, 128), (9, 2, 2, 256), (50, 4, 4, 8)])
