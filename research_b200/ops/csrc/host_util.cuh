@@ -95,6 +95,24 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// The driver's encoder needs a current context.  A thread that has made no runtime call that binds one (an autograd
+// thread whose first work is a product of this library) gets its device's primary context, and the call is made again.
+inline CUresult encode_tiled(EncodeTiledFn fn, CUtensorMap* out, CUtensorMapDataType dt, cuuint32_t rank,
+                             const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                             const cuuint32_t* box, CUtensorMapSwizzle swz) {
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  auto encode = [&] {
+    return fn(out, dt, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
+  return r;
+}
+
 // Rank-3 row-major tensor [d2][d1][d0] (d0 innermost) with byte strides s1 (between d1 rows) and
 // s2 (between d2 slabs); box {b0, b1, 1}; 128-byte swizzle; zero fill out of bounds.
 inline int make_map_3d(CUtensorMap* out, CUtensorMapDataType dt, const void* base, uint64_t d0, uint64_t d1,
@@ -106,9 +124,7 @@ inline int make_map_3d(CUtensorMap* out, CUtensorMapDataType dt, const void* bas
   cuuint64_t dims[3] = {d0, d1, d2 ? d2 : 1};
   cuuint64_t strides[2] = {s1_bytes, s2_bytes ? s2_bytes : s1_bytes * d1};
   cuuint32_t box[3] = {b0, b1, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(out, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = encode_tiled(fn, out, dt, 3, base, dims, strides, box, swz);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr,
             "research_b200: cuTensorMapEncodeTiled failed (%d) dims=(%llu,%llu,%llu) strides=(%llu,%llu) box=(%u,%u)\n",
@@ -128,9 +144,7 @@ inline int make_map_2d(CUtensorMap* out, CUtensorMapDataType dt, const void* bas
   cuuint64_t dims[2] = {d0, d1};
   cuuint64_t strides[1] = {s1_bytes};
   cuuint32_t box[2] = {b0, b1};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = encode_tiled(fn, out, dt, 2, base, dims, strides, box, swz);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr, "research_b200: cuTensorMapEncodeTiled(2d) failed (%d) dims=(%llu,%llu) stride=%llu box=(%u,%u)\n", (int)r,
             (unsigned long long)d0, (unsigned long long)d1, (unsigned long long)s1_bytes, b0, b1);
@@ -151,9 +165,7 @@ inline int make_map_4d(CUtensorMap* out, CUtensorMapDataType dt, const void* bas
   cuuint64_t dims[4] = {d0, d1, d2, d3};
   cuuint64_t strides[3] = {s1_bytes, s2_bytes, s3_bytes};
   cuuint32_t box[4] = {b0, b1, b2, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(out, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = encode_tiled(fn, out, dt, 4, base, dims, strides, box, swz);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr,
             "research_b200: cuTensorMapEncodeTiled(4d) failed (%d) dims=(%llu,%llu,%llu,%llu) strides=(%llu,%llu,%llu)\n",

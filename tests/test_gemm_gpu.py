@@ -271,3 +271,57 @@ def test_products_on_cta_pairs(M, N, K, ta, tb):
         native.check_status()
         # fp32 sums of K exact products: K * 2^-24 of the sum of magnitudes bounds any order
         assert (acc.double() - ref - 0.5).abs().max() <= K * 2.0 ** -24 * (size.max() + 1)
+
+
+def _in_new_thread(fn):
+    import threading
+
+    got = []
+
+    def work():
+        try:
+            got.append(fn())
+        except Exception as e:                      # noqa: BLE001 - handed to the test
+            got.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    return got[0]
+
+
+@pytest.mark.parametrize("product", ["gemm", "skinny", "attention"])
+def test_first_cuda_work_of_a_thread_can_be_a_product(product):
+    """A thread without a current CUDA context, whose first work encodes 3-, 2- and 4-dimensional tensor maps."""
+
+    from research_b200.ops import native
+
+    a, b = _rand((256, 256), 1), _rand((256, 256), 2)
+    q = _rand((1, 256, 2, 64), 3)
+    run = {"gemm": lambda: native.gemm(a, b), "skinny": lambda: native.gemm_skinny(a[:64], b),
+           "attention": lambda: native.attn_fwd(q, q, q)[0]}[product]
+    want = run()
+    got = _in_new_thread(run)
+    torch.cuda.synchronize()
+    native.check_status()
+    assert torch.is_tensor(got), got
+    assert torch.equal(got, want)
+
+
+def test_first_backward_of_a_process_can_start_with_a_product():
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    code = ("import torch\n"
+            "from research_b200.ops import functional as Fn, native\n"
+            "x = torch.randn(256, 256, device='cuda').bfloat16().requires_grad_(True)\n"
+            "w = torch.nn.Parameter(torch.randn(512, 256, device='cuda').bfloat16())\n"
+            "w.main_grad = torch.zeros(512, 256, device='cuda')\n"
+            "g = torch.ones(256, 512, device='cuda').bfloat16()\n"
+            "(dx,) = torch.autograd.grad([Fn.linear(x, w)], [x], [g])\n"
+            "native.check_status()\n"
+            "assert torch.allclose(dx.float(), w.float().sum(0).expand(256, 256), rtol=2e-2, atol=0.2)\n")
+    done = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, capture_output=True,
+                          text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
