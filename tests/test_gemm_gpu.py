@@ -325,3 +325,27 @@ def test_first_backward_of_a_process_can_start_with_a_product():
     done = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, capture_output=True,
                           text=True, timeout=300)
     assert done.returncode == 0, done.stderr
+
+
+def test_first_products_of_a_process_from_several_threads_at_once():
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    code = ("import threading, torch\n"
+            "from research_b200.ops import native\n"
+            "native.load(), native.status_word()\n"
+            "a = torch.ones(128, 128, device='cuda', dtype=torch.bfloat16)\n"
+            "gate, got = threading.Barrier(16), []\n"
+            "def work():\n"
+            "    gate.wait()\n"
+            "    try: got.append(native.gemm(a, a))\n"
+            "    except Exception as e: got.append(e)\n"
+            "threads = [threading.Thread(target=work) for _ in range(16)]\n"
+            "[t.start() for t in threads], [t.join() for t in threads]\n"
+            "torch.cuda.synchronize(), native.check_status()\n"
+            "assert all(torch.is_tensor(g) and (g == 128).all() for g in got), got\n")
+    for _ in range(3):
+        done = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, capture_output=True,
+                              text=True, timeout=300)
+        assert done.returncode == 0, done.stderr
