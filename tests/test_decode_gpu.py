@@ -220,6 +220,36 @@ def test_prompt_rows_in_pages(T, B, Hkv, D):
     assert not told._from_zero
 
 
+def _rows_laid_out(kind, B, T, H, D):
+    shape = {"time-major": (T, B, H, D), "one for all": (1, T, H, D), "padded sequences": (B, T * H * D + 8),
+             "padded rows": (B, T, H * D + 8), "every other row": (B, 2 * T, H, D), "head-major": (B, H, T, D)}[kind]
+    t = torch.randn(shape, device="cuda").bfloat16()
+    return {"time-major": lambda: t.transpose(0, 1), "one for all": lambda: t.expand(B, T, H, D),
+            "padded sequences": lambda: t[:, : T * H * D].view(B, T, H, D),
+            "padded rows": lambda: t[..., : H * D].view(B, T, H, D), "every other row": lambda: t[:, ::2],
+            "head-major": lambda: t.transpose(1, 2)}[kind]()
+
+
+@pytest.mark.parametrize("kind", ["time-major", "one for all", "padded sequences", "padded rows", "every other row", "head-major"])
+@pytest.mark.parametrize("B", [1, 3])
+def test_prompt_rows_wherever_they_lie(kind, B):
+    """The kernels read a prompt's rows in place where they can: the same as from contiguous copies, for every layout."""
+
+    from research_b200.infer.generation import PagedKVCache
+    from research_b200.ops import native
+
+    T, D = 130, 64
+    q, k, v = (_rows_laid_out(kind, B, T, h, D) for h in (4, 2, 2))
+    pos = torch.arange(T, device="cuda", dtype=torch.int32).expand(B, T).contiguous()
+    cache = PagedKVCache(layers=2, batch=B, max_len=T + 5, kv_heads=2, head_dim=D, page_size=128, dtype=torch.bfloat16,
+                         device=torch.device("cuda"))
+    o = cache.update_and_attend(1, q, k, v, pos, None)
+    want, _ = native.attn_fwd(q.contiguous(), k.contiguous(), v.contiguous())
+    native.check_status()
+    assert torch.equal(o, want.reshape(B, T, -1))
+    assert torch.equal(cache._rows(cache.k, 1, T), k) and torch.equal(cache._rows(cache.v, 1, T), v)
+
+
 # lengths around a page: fewer rows than one, a whole one, one row more
 @pytest.mark.parametrize("T", [2, 128, 129])
 def test_one_prompt_for_every_sequence_of_a_cache(T):

@@ -67,8 +67,9 @@ def _off(got, ref):
     return float((got.detach().double() - ref.detach().double()).norm() / ref.detach().double().norm())
 
 
-# widths on each side of the kernel's choices of columns per thread, rows around a block's group of rows
-@pytest.mark.parametrize("H", [256, 512, 768, 2048, 2560, 4096, 5632, 8192, 8200])
+# widths on each side of the kernel's choices of columns per thread (2304, 2816 and 3840 are multiples of 256 that take a
+# warp per row), rows around a block's group of rows
+@pytest.mark.parametrize("H", [256, 512, 768, 2048, 2304, 2560, 2816, 3840, 4096, 5632, 8192, 8200])
 @pytest.mark.parametrize("rows", [1, 5, 1203])
 @pytest.mark.parametrize("with_res", [False, True])
 def test_rmsnorm_bwd_widths(H, rows, with_res):

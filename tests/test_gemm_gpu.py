@@ -90,13 +90,13 @@ def test_skinny_splitk_gemm_matches_reference():
     from research_b200.ops import native
 
     torch.manual_seed(0)
-    # the shapes share one fp32 workspace that every call must leave zeroed: large after small and back again
+    # nothing is kept between calls: large after small and back again, each shape as often as it comes
     for rows, n, k in ((32, 2048, 2048), (32, 2048, 5632), (7, 11264, 2048), (64, 4096, 2048), (3, 512, 256),
                        (64, 11264, 2048), (32, 2048, 2048)):
         a = (torch.randn(rows, k, device="cuda") * 0.5).bfloat16()
         b = (torch.randn(n, k, device="cuda") * 0.05).bfloat16()
         ref = a.float() @ b.float().t()
-        for fused in (False, True):       # finishing pass as its own kernel / inside the product
+        for fused in (False, True):       # a switch of earlier callers: accepted, the result is the same
             y = native.gemm_skinny(a, b, fused_finish=fused)
             native.check_status()
             assert y.shape == (rows, n) and y.dtype == torch.bfloat16
@@ -271,6 +271,44 @@ def test_products_on_cta_pairs(M, N, K, ta, tb):
         native.check_status()
         # fp32 sums of K exact products: K * 2^-24 of the sum of magnitudes bounds any order
         assert (acc.double() - ref - 0.5).abs().max() <= K * 2.0 ** -24 * (size.max() + 1)
+
+
+# long enough for CTA pairs: contractions of uneven length, an empty one among them, with an output that has no whole
+# last tile; and K slices that pairs add into one output
+@pytest.mark.parametrize("m,n", [(2048, 2048), (2040, 1544)])
+def test_pair_products_with_ranges_of_k(m, n):
+    from research_b200.ops import native
+
+    torch.manual_seed(3)
+    ranges = [0, 4096, 4096, 4160, 8192, 12288]
+    a = (torch.randn(ranges[-1], m, device="cuda") * 0.1).bfloat16()
+    b = (torch.randn(ranges[-1], n, device="cuda") * 0.5).bfloat16()
+    assert ranges[-1] * m * n >= 2.5e10                      # the launcher's rule for pairs
+    out = torch.full((len(ranges) - 1, m, n), 0.25, device="cuda")
+    bounds = torch.tensor(list(zip(ranges[:-1], ranges[1:])), dtype=torch.int32, device="cuda")
+    rc = native.load().b200_gemm_bf16_grouped_k(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, ranges[-1], len(ranges) - 1, m, n, n, m * n, 1, 1,
+        bounds.data_ptr(), native.status_word().data_ptr(), native._stream())
+    assert rc == 0
+    native.check_status()
+    for i, (lo, hi) in enumerate(zip(ranges[:-1], ranges[1:])):
+        ad, bd = a[lo:hi].double(), b[lo:hi].double()
+        # exact products, fp32 sums of at most 4096 of them: the same bound as for one pass over 2999 tokens
+        assert (out[i].double() - 0.25 - ad.T @ bd).abs().max() <= 2.0 ** -18 * (ad.abs().T @ bd.abs()).max() + 2.0 ** -24, i
+
+
+def test_pair_products_with_slices_of_k():
+    from research_b200.ops import native
+
+    torch.manual_seed(4)
+    k, m, n = 4096, 2048, 5632
+    assert native.wave_splits(m, n, k) > 1 and k * m * n >= 2.5e10
+    dy, x = (torch.randn(k, m, device="cuda") * 0.1).bfloat16(), (torch.randn(k, n, device="cuda") * 0.5).bfloat16()
+    grad = torch.full((m, n), 0.25, device="cuda")
+    native.gemm_wgrad(dy, x, grad)
+    native.check_status()
+    ref, size = dy.double().T @ x.double(), dy.double().abs().T @ x.double().abs()
+    assert (grad.double() - 0.25 - ref).abs().max() <= 2.0 ** -18 * size.max() + 2.0 ** -24
 
 
 def _in_new_thread(fn):

@@ -4,6 +4,7 @@ import json
 import re
 from pathlib import Path
 
+import numpy as np
 import pytest
 import torch
 
@@ -212,3 +213,26 @@ def test_dependent_kernels_read_nothing_before_their_wait():
         reads = re.findall(r"tma_load_\w+|bulk_g2s|load8\w*|__ldg|\*reinterpret_cast<const", before)
         assert not reads, (name, reads)
     assert {"skinny_gemm_kernel", "qknorm_rope_fwd_kernel", "rmsnorm_fwd_row_kernel", "attn_bwd_kernel"} <= set(seen), seen
+
+
+def test_exponential_on_the_fma_pipes_keeps_its_stated_error():
+    """b200.cuh: f2_ex2 step by step in fp32, with the coefficients of the source, against 2^x in 64 bits."""
+
+    text = (build.PKG_ROOT / "ops" / "csrc" / "b200.cuh").read_text()
+    body = text[text.index("uint64_t f2_ex2("):]
+    body = body[:body.index("\n}")]
+    pairs = re.findall(r"f2_pack\((-?[\d.]+)f, \1f\)", body)
+    assert pairs[:3] == ["12582912.", "-12582912.", "-1."] and len(pairs) == 9, pairs
+    coefficients = [np.float32(c) for c in pairs[3:]]          # of f^5 down to 1
+    fma = lambda a, b, c: (a.astype(np.float64) * b + c).astype(np.float32)   # noqa: E731 - one rounding, as the device's
+    x = np.concatenate([np.linspace(-126, 126, 400_001), np.linspace(-2, 2, 400_001), [-1e30, -np.inf, 0.5, -0.5]]).astype(np.float32)
+    clamped = np.maximum(x, np.float32(-126))
+    t = clamped + np.float32(12582912.0)
+    f = fma(t + np.float32(-12582912.0), np.float32(-1), clamped)
+    p = np.full_like(f, coefficients[0])
+    for c in coefficients[1:]:
+        p = fma(p, f, c)
+    scale = ((t.view(np.int32) << 23) + np.int32(0x3F800000)).view(np.float32)
+    got, want = (p * scale).astype(np.float64), np.exp2(clamped.astype(np.float64))
+    error = np.abs(got / want - 1)
+    assert error.max() < 2.2e-7 and np.sqrt((error ** 2).mean()) < 8.5e-8, (error.max(), np.sqrt((error ** 2).mean()))

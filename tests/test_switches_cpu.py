@@ -105,3 +105,30 @@ def test_weight_gradients_are_one_pass_where_the_sums_have_to_repeat_themselves(
             native.gemm_wgrad(torch.zeros(k, m, dtype=torch.bfloat16), torch.zeros(k, n, dtype=torch.bfloat16),
                               torch.zeros(m, n))
     assert passes == [k for k in tokens for _ in range(3)]
+
+
+def test_kernels_go_without_their_autograd_function_only_where_nothing_records_or_transforms():
+    from torch.autograd import forward_ad
+
+    seen = {}
+
+    def look(name):
+        def fn(t):
+            seen[name] = Fn._no_derivatives()
+            return t.sum()
+        return fn
+
+    x = torch.ones(2, 3)
+    look("grad mode")(x)
+    with torch.no_grad():
+        look("no_grad")(x)
+        torch.func.vmap(look("vmap"))(x)
+        torch.func.grad(look("grad"))(x)
+        torch.func.jvp(look("jvp"), (x,), (x,))
+        with forward_ad.dual_level():
+            look("forward mode")(forward_ad.make_dual(x, x))
+        look("after")(x)
+    with torch.inference_mode():
+        look("inference mode")(x)
+    assert seen == {"grad mode": False, "no_grad": True, "vmap": False, "grad": False, "jvp": False,
+                    "forward mode": False, "after": True, "inference mode": True}
