@@ -63,7 +63,8 @@ inline int ensure_dynamic_smem(Kern* kern, int bytes, bool (&done)[kMaxDevices])
   return 0;
 }
 
-// RESEARCH_B200_PDL=0 turns programmatic dependent launch off for the kernels of a decode step that use it.
+// RESEARCH_B200_PDL=0 turns programmatic dependent launch off: for the kernels of a decode step that use it, and for the
+// two kernels of the attention backward, which then run one after the other.
 inline int pdl_enabled() {
   static const int on = [] {
     const char* v = getenv("RESEARCH_B200_PDL");

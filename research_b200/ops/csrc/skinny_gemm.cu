@@ -8,9 +8,9 @@
 //   warp 1     MMA issuer: D[n][token] += W x^T in tensor memory
 //   warps 2-5  move the partial D to shared memory, token by token
 // The CTAs of a cluster then each sum 128 / cluster rows of D over all partials, read from one another's shared memory in
-// rank order, and write bf16: no workspace, no finishing kernel, the same bits every time.  Slices that added into an
-// fp32 workspace with reduce-adds and a kernel that converted it and cleared it behind itself took @OLD@ where this takes
-// @NEW@.
+// rank order, and write bf16: no workspace, no finishing kernel, the same bits every time.  The four linears of a
+// 2048-wide layer (wqkv, wo, w_gate_up, w_down) with 32 rows: 45 us as slices added into an fp32 workspace with
+// reduce-adds and a kernel that converted it and cleared it, 32.4 us here; 28.3 us with one row.
 #include "b200.cuh"
 #include "host_util.cuh"
 
@@ -206,12 +206,12 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 template <int NT>
 int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyParams p, int grid, cudaStream_t stream) {
   auto* kern = skinny_gemm_kernel<NT>;
-  // The ring takes what the CTAs that share an SM leave each other (up to three): 10 stages for one CTA, 3 for three.
-  // 2048 x 5632 with 32 rows, 128 CTAs: 11.7 us with 3 stages, 8.0 with 5; 50304 x 2048, 393 CTAs: 38.0 us with 5
-  // (two a SM), 33.8 with 3 (three a SM).
+  // The ring takes what the CTAs that share an SM leave each other: with 16 / 32 / 64 / 128 rows 12 / 11 / 9 / 7 stages
+  // for one CTA, 6 / 5 / 4 / 3 for two and 4 / 3 / 3 / 2 for three.  32 rows, rings for one, two and three CTAs an SM:
+  // 11264 x 2048, 88 CTAs 11.5 / 12.5 / 14.9 us; 50304 x 2048, 393 CTAs 39.2 / 37.8 / 33.8 us.
   const int sms = b200host::sm_count();
   int per_sm = grid <= sms ? 1 : (grid <= 2 * sms ? 2 : 3);
-  // eight CTAs on eight SMs to themselves do not fit every part of the device at once (2048 x 5632: 11.2 us, 8.0 with room
+  // eight CTAs on eight SMs to themselves do not fit every part of the device at once (2048 x 5632: 12.6 us, 7.9 with room
   // for two on an SM)
   if (p.cluster == 8 && per_sm == 1) per_sm = 2;
   const int budget = (226 * 1024 / per_sm - 2048) / stage_bytes<NT>();

@@ -352,8 +352,8 @@ def splitk_factor(n: int, k: int, sms: int = 148) -> int:
     """Slices of K (1, 2, 4 or 8 CTAs of a cluster) for a skinny ``[rows, k] x [n, k]^T`` product: the count of least
     estimated time, the larger of what the busiest SM streams (0.27 us per 16 KB block of a 128-row tile) and of the
     whole matrix at 6.3 TB/s, plus the exchange of partial sums.  Slices are at least two blocks.  Measured with 32
-    rows: 4096 x 2048 1 / 2 / 4 / 8 slices 7.8 / 6.8 / 6.4 / 7.0 us, 2048 x 5632 16.4 / 10.0 / 8.3 / 8.0 us, 11264 x 2048
-    10.9 / 12.0 / 11.2 / 16.6 us, 6144 x 4096 13.6 / 11.8 / 12.4 / 12.7 us, 50304 x 2048 34 / 41 / 48 / 65 us."""
+    rows: 4096 x 2048 1 / 2 / 4 / 8 slices 8.2 / 7.2 / 6.8 / 7.6 us, 2048 x 5632 15.6 / 10.2 / 8.3 / 7.9 us, 11264 x 2048
+    11.5 / 12.6 / 11.4 / 17.3 us, 6144 x 4096 14.3 / 12.2 / 12.9 / 13.0 us, 50304 x 2048 34 / 39 / 46 / 69 us."""
 
     tiles, blocks = (n + 127) // 128, k // 64
     best, best_cost = 1, float("inf")
