@@ -17,7 +17,7 @@
 // maximum takes three operands an instruction, the scaling and the sum two lanes, and the loop bounds that select
 // descriptors are made warp-uniform (b200.cuh: warp_uniform).  With P in shared memory, a pass for the maximum and
 // descriptors in ordinary registers the loop took 6100 clocks: 8 x 4096 tokens of 16 / 8 heads of 128, causal, 782 us,
-// now 548 (703 -> 1004 TFLOP/s); 16384 tokens 1382 us, now 898 (1224 TFLOP/s).  A quarter of the exponentials as
+// now 536 to 556 by box; 16384 tokens 1382 us, now 898 to 1050 by the clock under power.  A quarter of the exponentials as
 // polynomials on the FMA pipes made it slower (920 us).
 // Masks: every query row attends to kv positions in [lo[row], row] (causal) or [lo[row], S) (not
 // causal); `lo` (int32 [B,S], non-decreasing along S, optional) encodes document starts and sliding
